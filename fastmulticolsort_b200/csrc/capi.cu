@@ -95,6 +95,10 @@ int sort_round_dev(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, uint32_
 {
     int rc;
     void *p;
+    // The keys of one-row segments are not needed when only the boundary scan
+    // below reads them: such a row and the row after it start a group whatever
+    // their keys, because in_group differs there.
+    const bool keys_scratch = !keys_out && in_group;
     if (!keys_out) {
         if ((rc = ws_get(ctx, kSlotKeys0, n * bank_bytes, &p))) return rc;
         keys_out = p;
@@ -121,6 +125,7 @@ int sort_round_dev(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, uint32_
     a.n = n;
     a.fixed_launches = fixed_launches;
     a.top_hist = in_group ? nullptr : top_hist;
+    a.keys_scratch = keys_scratch;
     if ((rc = sort_segments(ctx, a))) return rc;
     if (out_group || next_seg_start)
         return launch_group_ids_segments(ctx, keys_out, bank_bytes, in_group, out_group, next_seg_start, n,

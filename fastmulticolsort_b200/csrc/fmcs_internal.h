@@ -234,6 +234,9 @@ struct SortArgs {
     // says the rows are in order already (every segment is only copied).
     const uint32_t *d_key_bits = nullptr;
     const uint32_t *d_in_order = nullptr;
+    // The caller uses keys_out only to find the boundaries inside the segments
+    // it passed in: the key of a one-row segment need not be written.
+    bool keys_scratch = false;
 };
 int sort_segments(fmcs_ctx *ctx, const SortArgs &a);
 // Rows per look-back chunk of an HBM radix level (kChunkTiles tiles of the

@@ -305,7 +305,8 @@ __device__ __forceinline__ int route_segment(uint32_t start, uint32_t len, uint3
 template <typename K>
 __global__ void classify_kernel(Bufs<K> b, const uint32_t *__restrict__ seg_start, const uint32_t *d_nseg,
                                 uint64_t n, uint32_t key_bits, uint32_t *ctr, LargeSeg *large0, Lists lists,
-                                const uint32_t *top_hist, const uint32_t *d_key_bits, const uint32_t *d_in_order)
+                                const uint32_t *top_hist, const uint32_t *d_key_bits, const uint32_t *d_in_order,
+                                bool skip_single)
 {
     kernel_prologue();
     if (d_key_bits) key_bits = min(key_bits, *d_key_bits);
@@ -326,7 +327,13 @@ __global__ void classify_kernel(Bufs<K> b, const uint32_t *__restrict__ seg_star
         const uint32_t end = seg_start ? seg_start[s + 1] : (uint32_t)n;
         const uint32_t len = end - start;
         if (len == 1) {
-            // A one-row segment keeps its position: copy it straight to BUF0.
+            // A one-row segment keeps its position.  With skip_single its oid
+            // is in BUF0 already and nothing reads its key: nothing to do.
+            // (Fetching those keys was a random 32-byte sector per row: 1.25 ms
+            // of the second round of a 67M-row plan whose first round leaves
+            // one-row groups, against 0.06 ms for reading the segment starts.)
+            if (skip_single) continue;
+            // Otherwise copy it straight to BUF0.
             K k;
             uint32_t v;
             load_kv(b, kSrcExt, start, k, v);
@@ -1665,7 +1672,8 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
         if (seg_start && a.nseg_host == 0) grid = (unsigned)sms * 16;
         { LaunchScope ls_(ctx, "classify");
             launch_k(classify_kernel<K>, grid, 256, 0, st, b, seg_start, d_nseg, n, a.key_bits, ctr, large[0], lists,
-                     seg_start ? nullptr : a.top_hist, a.d_key_bits, a.d_in_order);
+                     seg_start ? nullptr : a.top_hist, a.d_key_bits, a.d_in_order,
+                     a.keys_scratch && a.order_in == a.order_out);
         }
         FMCS_LAUNCH_CHECK("classify");
     }
