@@ -168,8 +168,10 @@ int join_par(fmcs_ctx *ctx, cudaStream_t st);
 // begin launching while the stream's previous kernel finishes (its prologue
 // waits for that kernel's completion).  Every kernel launched this way starts
 // with kernel_prologue().
+// early == false: an ordinary launch, after the previous kernel has left the GPU.
 template <typename... P, typename... A>
-inline cudaError_t launch_k(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args)
+inline cudaError_t launch_on(bool early, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                             A &&...args)
 {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -180,8 +182,13 @@ inline cudaError_t launch_k(void (*k)(P...), dim3 grid, dim3 block, size_t smem,
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_k(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args)
+{
+    return launch_on(true, k, grid, block, smem, st, std::forward<A>(args)...);
 }
 
 // True when the device can dereference p directly (device or managed memory).

@@ -39,3 +39,48 @@ def test_one_row_segments(ctx, pattern, dtype, bits, want_keys):
     ctx.sort_round(stale, bits, np.zeros(n, np.uint32), out_group=np.zeros(n, np.uint32))
     bank = (rng.integers(0, 1 << 16, size=n, dtype=np.uint64) % 5 + 5).astype(dtype)
     _segmented(ctx, sizes, bank, bits, 11, want_keys)
+
+
+# segment sizes on both sides of every on-chip capacity (and of the powers of
+# two that set the bucket count)
+EDGES = [2, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025, 2047,
+         2048, 2049, 2304, 2305, 4095, 4096, 4097, 8191, 8192]
+
+
+def _bank(kind, n, bits, rng):
+    top = (1 << bits) - 1
+    if kind == "uniform":
+        return rng.integers(0, top, size=n, dtype=np.uint64, endpoint=True)
+    if kind == "few":        # a handful of values: many equal keys
+        return rng.integers(0, 3, size=n, dtype=np.uint64) * np.uint64(top // 2)
+    if kind == "skewed":     # one leading code holds most rows, the rest of the key spreads
+        lead = bits // 3
+        hot = rng.random(n) < 0.9
+        lead_code = np.where(hot, 1, rng.integers(0, 1 << lead, size=n, dtype=np.uint64)).astype(np.uint64)
+        return (lead_code << np.uint64(bits - lead)) | rng.integers(0, 1 << (bits - lead), size=n, dtype=np.uint64)
+    # "ends": differences in the highest and the lowest bit only
+    return (rng.integers(0, 2, size=n, dtype=np.uint64) << np.uint64(bits - 1)) | rng.integers(0, 2, size=n,
+                                                                                               dtype=np.uint64)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "few", "skewed", "ends"])
+@pytest.mark.parametrize("dtype,bits", [(np.uint16, 16), (np.uint32, 32), (np.uint64, 51), (np.uint64, 52),
+                                        (np.uint64, 64)])
+def test_onchip_segments(ctx, kind, dtype, bits):
+    """Bucketing by digit and by splitters, compounds that fit 64 bits (51 key
+    bits and 13 position bits) and that do not."""
+    rng = np.random.default_rng(bits + len(kind))
+    sizes = [int(s) for s in rng.permutation(EDGES * 2)]
+    bank = _bank(kind, int(np.sum(sizes)), bits, rng).astype(dtype)
+    _segmented(ctx, sizes, bank, bits, 5, want_keys=True)
+
+
+@pytest.mark.parametrize("n", EDGES)
+@pytest.mark.parametrize("kind", ["skewed", "few"])
+def test_onchip_whole_round(ctx, n, kind):
+    rng = np.random.default_rng(n)
+    bank = _bank(kind, n, 64, rng)
+    order, group = np.zeros(n, np.uint32), np.zeros(n, np.uint32)
+    ng = ctx.sort_round(bank, 64, order, out_group=group)
+    o, g, _, ng_ref = O.sort_round(bank)
+    assert ng == ng_ref and np.array_equal(order, o) and np.array_equal(group, g)
