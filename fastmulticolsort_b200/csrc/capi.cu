@@ -167,7 +167,7 @@ int plan_pipeline(fmcs_ctx *ctx, const Plan &plan, const void *const *dcols, con
     // (a) a bank's stitch reads only the columns: the next round's bank is
     // stitched on the context's second stream while this round sorts (its
     // buffer held the bank of the round before, finished by then)
-    const uint32_t chunk_rows = msd_chunk_rows(ctx);
+    const uint32_t chunk_rows = msd_chunk_rows(ctx, n);
     uint32_t *top_hist = nullptr;
     auto stitch_bank = [&](uint32_t b, cudaStream_t s, void **bank_out) -> int {
         const BankPlan &bp = plan.banks[b];
@@ -185,7 +185,8 @@ int plan_pipeline(fmcs_ctx *ctx, const Plan &plan, const void *const *dcols, con
         if (!hash && b == 0 && n > ctx->local_max) {
             const uint64_t nchunks = (n + chunk_rows - 1) / chunk_rows;
             void *q;
-            if ((r = ws_get(ctx, kSlotTopHist, (nchunks + 1) * 256 * sizeof(uint32_t), &q))) return r;
+            if ((r = ws_get(ctx, kSlotTopHist, (nchunks + (nchunks + kTopSuper - 1) / kTopSuper) * 256 * sizeof(uint32_t), &q)))
+                return r;
             th = (uint32_t *)q;
             top_hist = th;
         }
@@ -859,13 +860,10 @@ static int graph_create(fmcs_ctx *parent, const void *const *cols, const uint32_
     // 1) one eager run of the fixed launch sequence sizes every workspace slot
     rc = plan_pipeline(ctx, plan, cols, col_bytes, bw, n, hash, order_out, group_out, true, &g->d_ng);
     if (!rc) rc = check_status(ctx, "fmcs_graph_create warm-up");
-    // 2) capture: reset the look-back words (their epochs repeat on every
-    //    replay), then the same launches
+    // 2) capture the same launches
     if (!rc) {
         cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            for (int slot : {kSlotLookback, kSlotScanTiles})
-                if (ctx->ws.ptr[slot]) cudaMemsetAsync(ctx->ws.ptr[slot], 0, ctx->ws.cap[slot], ctx->stream);
             const unsigned long long l0 = ctx->launches;   // every launch site counts itself
             rc = plan_pipeline(ctx, plan, cols, col_bytes, bw, n, hash, order_out, group_out, true, &g->d_ng);
             g->kernels = ctx->launches - l0;

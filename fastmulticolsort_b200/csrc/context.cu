@@ -28,7 +28,7 @@ int cuda_fail(fmcs_ctx *ctx, cudaError_t e, const char *what)
     return set_error(ctx, e == cudaErrorMemoryAllocation ? FMCS_E_OOM : FMCS_E_CUDA, buf);
 }
 
-int ws_get(fmcs_ctx *ctx, int slot, size_t bytes, void **out, bool zero_new)
+int ws_get(fmcs_ctx *ctx, int slot, size_t bytes, void **out)
 {
     Workspace &w = ctx->ws;
     if (bytes == 0) bytes = 256;
@@ -60,15 +60,6 @@ int ws_get(fmcs_ctx *ctx, int slot, size_t bytes, void **out, bool zero_new)
     if (e != cudaSuccess) {
         cudaGetLastError();
         return cuda_fail(ctx, e, "workspace cudaMalloc");
-    }
-    if (zero_new) {
-        // look-back words must not carry a stale (epoch, flag) from whatever
-        // the allocation held before
-        e = cudaMemsetAsync(p, 0, want, ctx->stream);
-        if (e != cudaSuccess) {
-            cudaFree(p);
-            return cuda_fail(ctx, e, "workspace memset");
-        }
     }
     w.ptr[slot] = p;
     w.cap[slot] = want;
@@ -441,8 +432,8 @@ extern "C" long long fmcs_get_tuning(const fmcs_ctx *ctx, const char *key)
 }
 
 // ---------------------------------------------------------------------------
-// Self-test of the bounded device waits: one warp waits, through lb_wait (the
-// wait every look-back of the library uses), on a word of the workspace that
+// Self-test of the bounded device wait: one warp waits, through lb_wait (the
+// only way the library's device code waits), on a word of the workspace that
 // no kernel writes.  The wait must give up after `polls` polls, record
 // FMCS_E_TIMEOUT in the context's status word and return, leaving the
 // context usable.

@@ -1,9 +1,9 @@
 // device_common.cuh -- device helpers shared by the sm_100a kernels of the
-// multi-column sort path: typed key access, radix digits, warp-level
-// multi-split ranking (match.any + ballot), and the bounded waits used by the
-// decoupled look-back scans (every wait has an iteration limit, after which the
-// kernel records FMCS_E_TIMEOUT in a device status word and carries on, so a
-// lost predecessor can never hang the GPU).
+// multi-column sort path: radix digits, warp-level multi-split ranking
+// (match.any, ballots or shared-memory OR words), and a bounded wait: it has an
+// iteration limit, after which the kernel records FMCS_E_TIMEOUT in a device
+// status word and carries on, so that it can never hang the GPU.  (No kernel
+// of the sort path waits for another block; the self-test runs the wait.)
 #pragma once
 
 #include <cstdint>
@@ -20,8 +20,7 @@ constexpr int kDevOk = 0;
 constexpr int kDevTimeout = -3;
 constexpr int kDevBadInput = -1;
 
-// Look-back words: hi 32 bits = (epoch << 2) | flag, lo 32 bits = value.
-constexpr uint32_t kFlagAggregate = 1;
+// Words that a wait polls: hi 32 bits = (epoch << 2) | flag, lo 32 bits = value.
 constexpr uint32_t kFlagInclusive = 2;
 // A wait gives up after this many polls (with nanosleep back-off that is well
 // over a second; a healthy predecessor publishes within microseconds).
@@ -59,11 +58,6 @@ __device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned lon
     unsigned long long v;
     asm volatile("ld.volatile.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
-}
-
-__device__ __forceinline__ void st_volatile_u64(unsigned long long *p, unsigned long long v)
-{
-    asm volatile("st.volatile.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 __device__ __forceinline__ unsigned long long lb_word(uint32_t epoch, uint32_t flag, uint32_t value)
@@ -217,7 +211,7 @@ __device__ __forceinline__ void block_exclusive_scan_radix(uint32_t *cnt, uint32
     __syncthreads();
 }
 
-// Bounded wait on a look-back word of the given epoch.  Returns the word, or 0
+// Bounded wait on a word of the given epoch.  Returns the word, or 0
 // after recording a timeout in *status (the caller treats 0 as an inclusive
 // value of 0 so that every waiter still finishes).  `limit` polls at most.
 __device__ __forceinline__ unsigned long long lb_wait(const unsigned long long *p, uint32_t epoch,

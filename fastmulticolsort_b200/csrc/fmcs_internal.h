@@ -28,12 +28,11 @@ enum Slot : int {
     kSlotLarge1,      // large-segment descriptors, pong
     kSlotSegHist,     // per large segment digit histograms / offsets
     kSlotTilePrefix,  // tile prefix per large segment
-    kSlotLookback,    // look-back words
     kSlotLocalA,      // local lists, warp tier
     kSlotLocalB,      // block tier (medium)
     kSlotLocalC,      // block tier (large)
     kSlotCounters,    // small device counters
-    kSlotScanTiles,   // look-back words of the flag scans
+    kSlotScanTiles,   // per-tile counts and masks of the boundary scans
     kSlotHashTable,   // hash grouping table
     kSlotHashIdx,     // hash grouping per-row ids
     kSlotStageIn0,    // host-staging buffers
@@ -82,7 +81,6 @@ struct fmcs_ctx {
     size_t held = 0;     // bytes held by the workspace
     fmcs::Workspace ws;
     int *d_status = nullptr;       // device status word
-    uint32_t epoch = 1;            // look-back epoch, advanced per launch
     std::string err;
     int *h_status = nullptr;       // pinned mirror of the status word
     uint32_t *h_small = nullptr;   // pinned small read-back area (64 words)
@@ -132,7 +130,7 @@ class Carver {
 int set_error(fmcs_ctx *ctx, int code, const std::string &msg);
 int cuda_fail(fmcs_ctx *ctx, cudaError_t e, const char *what);
 // Returns a device pointer of at least `bytes` in `slot` (grown as needed).
-int ws_get(fmcs_ctx *ctx, int slot, size_t bytes, void **out, bool zero_new = false);
+int ws_get(fmcs_ctx *ctx, int slot, size_t bytes, void **out);
 // Checks and clears the device status word (synchronizes the stream).
 int check_status(fmcs_ctx *ctx, const char *what);
 
@@ -203,11 +201,11 @@ struct StitchSlice {
     uint32_t invert;   // 1: the slice's bits are inverted (its column sorts descending)
 };
 constexpr int kMaxSlices = 32;
-// With top_hist (device, 256 words per chunk of chunk_rows rows and one more
-// row), the stitch also counts the top digit (bits [key_bits - min(8,
-// key_bits), key_bits)) of every bank value, one row per chunk and the total
-// in the last row: the first radix level's histograms of a round-0 sort of
-// the bank (chunk_rows = msd_chunk_rows).
+// With top_hist (device, 256 words per chunk of chunk_rows rows, then 256 per
+// kTopSuper chunks), the stitch also counts the top digit (bits [key_bits -
+// min(8, key_bits), key_bits)) of every bank value, one row per chunk and then
+// the sums of every kTopSuper of them: the first radix level's histograms of a
+// round-0 sort of the bank (chunk_rows = msd_chunk_rows).
 // `stream`: NULL for the context's stream.
 int launch_stitch(fmcs_ctx *ctx, const StitchSlice *sl, int ns, void *bank, uint32_t bank_bytes,
                   uint64_t n, uint32_t *top_hist = nullptr, uint32_t key_bits = 0, uint32_t chunk_rows = 0,
@@ -246,9 +244,11 @@ struct SortArgs {
     bool keys_scratch = false;
 };
 int sort_segments(fmcs_ctx *ctx, const SortArgs &a);
-// Rows per look-back chunk of an HBM radix level (kChunkTiles tiles of the
+// Rows per chunk of an HBM radix level of a round of n rows (tiles of the
 // context's tile size): the row granularity of the per-chunk histograms.
-uint32_t msd_chunk_rows(const fmcs_ctx *ctx);
+uint32_t msd_chunk_rows(const fmcs_ctx *ctx, uint64_t n);
+// The stitch writes super rows (sums of kTopSuper chunk rows) after the chunks'.
+constexpr uint32_t kTopSuper = 32;
 // Stable full-array LSD radix sort of (keys, vals) in place by key bits
 // [0, bits): the plain, unsegmented comparator path.
 int lsd_sort_full(fmcs_ctx *ctx, void *keys, uint32_t key_bytes, uint32_t *vals, uint64_t n, uint32_t bits);

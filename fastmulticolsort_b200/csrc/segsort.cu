@@ -12,10 +12,10 @@
 //   len <= 16 (32)  one thread per segment, rows in registers;
 //   len <= 256      one warp per segment, on chip;
 //   len <= 8192     one CTA per segment, on chip;
-//   larger          MSD radix levels: per-segment digit histogram, then a
-//                   onesweep-style stable scatter with a decoupled look-back
-//                   chained over the segment's tiles; every non-empty bucket
-//                   becomes a child segment with 8 bits fewer, re-binned.
+//   larger          MSD radix levels: digit histograms per chunk of a segment,
+//                   their prefixes, then a stable scatter without waits; every
+//                   non-empty bucket becomes a child segment with 8 bits
+//                   fewer, re-binned.
 // The MSD scatter ranks keys by warp-level multi-split, so every pass is
 // stable, and the on-chip sorts decide ties by position: the whole sort is
 // stable, ties keep the oid order of the input, which is what the reference
@@ -60,7 +60,7 @@ constexpr int kHistCtas = 4;         // resident histogram CTAs per SM (the grid
 constexpr int kMsdCtas16 = 3;       // resident scatter CTAs per SM with 16 rows per thread
 
 // counters slot words
-constexpr int kCtrMsdTile = 1;
+constexpr int kCtrMsdTile = 1;      // the scatter's next chunk
 constexpr int kCtrLarge0 = 2;   // + level parity
 constexpr int kCtrLocalA = 4;
 constexpr int kCtrLocalA2 = 20;
@@ -78,28 +78,40 @@ constexpr uint32_t kCopySplit = 4096;
 constexpr int kCtrLevel = 15;      // MSD levels started so far (device-side level index)
 constexpr int kCtrLocalC3 = 16;
 constexpr int kCtrLocalC1b = 17;
-constexpr int kCtrChunks0 = 18;    // + level parity: histogram rows (chunks) of the level's large segments
+constexpr int kCtrWork = 18;       // chunks the current level's scatter moves
+constexpr int kCtrLong = 19;       // super rows of the level's long segments (level_prefix_kernel)
 constexpr int kCtrWords = 32;
 
-// An HBM level cuts each large segment's look-back chain every kChunkTiles
-// tiles.  Each chunk has its own histogram row; msd_plan turns the rows of a
-// segment into per-chunk digit bases (the segment's offset of the digit plus
-// the digit's rows in the segment's earlier chunks), so a chunk's first tile
-// publishes its inclusive prefix at once and no tile walks back past its
-// chunk's start.  One long chain (a round's single segment of thousands of
-// tiles) makes every tile wait on the whole GPU's progress; short chains run
-// side by side (one level over 16.8M rows: 0.164 ms as one segment, 0.137 ms
-// as 256 segments of 16 tiles).  Chunks of 32 tiles keep most of that gain
-// (the scatter 3 us slower per step than with 16) and halve the rows the
-// plan walks (8 us faster).
-constexpr uint32_t kChunkTiles = 32;
+// An HBM level cuts each large segment into chunks of a few tiles (chunk_rows
+// rows, msd_chunk_rows).  A chunk has its own histogram row, counted by the CTA
+// that reads it; msd_plan turns the rows of a segment into absolute digit bases
+// (where the chunk's rows of a digit go), so the scatter's CTAs wait for
+// nothing: a CTA takes a chunk and moves its tiles one after the other, its
+// digit bases running on in registers.  Every kSuper chunks of a segment also
+// share a super row, the sum of theirs, so that no plan CTA walks more than
+// kSuper chunk rows and a few super rows.
+// Chunk size: one tile as long as there are no more than 32,768 (each is flushed
+// and planned).  Larger chunks cost: the scatter's last round over its 444
+// resident CTAs is as long as a chunk, and neighbouring tiles, whose rows share
+// the ends of every digit's run, are then written far apart in time, so that
+// half-filled lines leave L2 (16.8M rows: a level 108 us with one tile a
+// chunk, 132 with two, 148 with five and 190 MB read instead of 134; a 67M-row
+// Zipf plan 3.43 ms with one, 3.55 with two, 3.68 with four).
+constexpr uint64_t kChunksWanted = 16384;
+constexpr uint32_t kSuper = kTopSuper;
 
 struct LargeSeg {
     uint32_t start, len, shift, src;
 };
 
+// A chunk to scatter: rows [start, start + len) of a segment, its histogram
+// row, and the segment's remaining key bits and source (shift | src << 8).
+struct Chunk {
+    uint32_t start, len, row, info;
+};
+
 // The two alternating sets of an MSD level's buffers (large-segment list and
-// digit histogram rows; level L reads set L & 1 and fills set (L + 1) & 1).
+// the segments' digit totals; level L reads set L & 1 and fills set (L + 1) & 1).
 // With dev_level the level index is read on the device (ctr[kCtrLevel]), so a
 // level's launches are the same for every level (one graph body that loops);
 // otherwise every launch works on set 0.
@@ -107,23 +119,30 @@ struct LargeSeg {
 // parity: a parameter array indexed at run time is copied to local memory.)
 struct LevelRefs {
     LargeSeg *large[2];
-    uint32_t *hist[2];
+    uint32_t *super[2];       // kRadix words per super row (super_row)
+    uint32_t *hist;           // kRadix words per chunk: its rows by digit, then its digit bases
+    uint32_t *chunk_prefix;   // per large segment, its first chunk (level_prefix_kernel)
+    uint2 *long_rows;         // (segment, super row of it) of the segments of more than kSuper chunks
+    Chunk *work;              // the chunks to scatter (msd_plan)
     uint32_t *ctr;
+    uint32_t chunk_rows, max_chunks;   // max_chunks: n / chunk_rows
     int dev_level;
-    int hist0_ready;   // level 0's histogram was counted before the sort (by the stitch)
-    // Per large segment, its first histogram row (chunk), prefix-summed by
-    // level_prefix_kernel; NULL: one row and one look-back chain per segment.
-    uint32_t *chunk_prefix;
-    // With hist0_ready: level 0's per-chunk histogram rows as the stitch
-    // counted them, and after them the segment's total row (msd_plan reads
-    // them and writes the bases to hist[0]).
+    // level 0 (one segment) was counted before the sort, by the stitch: its
+    // chunks' rows and after them their super rows
     const uint32_t *top_hist;
 };
 
-__host__ __device__ __forceinline__ uint32_t seg_chunks(uint32_t len, uint32_t tile_rows)
+// The first super row of segment s, whose first chunk is c0.  (Rounding c0
+// down and counting the segments before it leaves room for every segment's.)
+__device__ __forceinline__ uint32_t super_row(uint32_t c0, uint32_t s) { return c0 / kSuper + s; }
+// Super rows of a level of nseg segments, at most.
+__host__ __device__ __forceinline__ uint64_t super_rows_max(uint64_t max_chunks, uint64_t nseg)
 {
-    const uint32_t tiles = (len + tile_rows - 1) / tile_rows;
-    return (tiles + kChunkTiles - 1) / kChunkTiles;
+    return (max_chunks + nseg) / kSuper + nseg + 1;
+}
+__host__ __device__ __forceinline__ uint32_t seg_chunks(uint32_t len, uint32_t chunk_rows)
+{
+    return (len - 1) / chunk_rows + 1;   // len >= 1
 }
 
 // Index of the level whose launches are running (level_prefix_kernel has
@@ -159,13 +178,6 @@ __device__ __forceinline__ void load_kv(const Bufs<K> &b, uint32_t src, uint64_t
         k = b.k0[i];
         v = b.v0[i];
     }
-}
-
-template <typename K>
-__device__ __forceinline__ K load_k(const Bufs<K> &b, uint32_t src, uint64_t i)
-{
-    if (src == kSrcExt) return b.ext_order ? b.ext_bank[b.ext_order[i]] : b.ext_bank[i];
-    return src == kSrcBuf1 ? b.k1[i] : b.k0[i];
 }
 
 // A segment's rows into registers: warp-striped positions wbase + j*32 + lane
@@ -238,12 +250,8 @@ __device__ __forceinline__ uint32_t alloc_slot(uint32_t *ctr, int which)
     return base + __popc(peers & lanemask_lt());
 }
 
-// A large segment gets its next-level histogram row zeroed here when
-// hist_out is given (the round's initial segments); the children of a radix
-// level get theirs zeroed by that level's scatter grid, coalesced.
 __device__ __forceinline__ int route_segment(uint32_t start, uint32_t len, uint32_t shift, uint32_t src,
-                                             uint32_t *ctr, int large_ctr, LargeSeg *large_out, const Lists &L,
-                                             uint32_t *hist_out)
+                                             uint32_t *ctr, int large_ctr, LargeSeg *large_out, const Lists &L)
 {
     if (len == 0) return -1;
     int which;
@@ -290,14 +298,7 @@ __device__ __forceinline__ int route_segment(uint32_t start, uint32_t len, uint3
     case kCtrLocalC1b: L.c1b[slot] = e; break;
     case kCtrLocalC2: L.c2[slot] = e; break;
     case kCtrLocalC3: L.c3[slot] = e; break;
-    default: {
-        large_out[slot] = LargeSeg{start, len, shift, src};
-        if (hist_out) {
-            uint4 *row = reinterpret_cast<uint4 *>(hist_out + (uint64_t)slot * kRadix);
-#pragma unroll 4
-            for (int i = 0; i < kRadix / 4; ++i) row[i] = make_uint4(0, 0, 0, 0);
-        }
-    }
+    default: large_out[slot] = LargeSeg{start, len, shift, src};
     }
     return which;
 }
@@ -308,8 +309,8 @@ __device__ __forceinline__ int route_segment(uint32_t start, uint32_t len, uint3
 template <typename K>
 __global__ void classify_kernel(Bufs<K> b, const uint32_t *__restrict__ seg_start, const uint32_t *d_nseg,
                                 uint64_t n, uint32_t key_bits, uint32_t *ctr, LargeSeg *large0, Lists lists,
-                                const uint32_t *top_hist, const uint32_t *d_key_bits, const uint32_t *d_in_order,
-                                bool skip_single)
+                                const uint32_t *top_hist, const uint32_t *d_key_bits,
+                                const uint32_t *d_in_order, bool skip_single)
 {
     kernel_prologue();
     if (d_key_bits) key_bits = min(key_bits, *d_key_bits);
@@ -344,19 +345,19 @@ __global__ void classify_kernel(Bufs<K> b, const uint32_t *__restrict__ seg_star
             b.v0[start] = v;
             continue;
         }
-        // (level 0's histogram rows are zeroed by its level_prefix_kernel)
-        route_segment(start, len, key_bits, kSrcExt, ctr, kCtrLarge0, large0, lists, nullptr);
+        route_segment(start, len, key_bits, kSrcExt, ctr, kCtrLarge0, large0, lists);
     }
 }
 
 // ---------------------------------------------------------------------------
 // MSD level kernels (large segments)
 // ---------------------------------------------------------------------------
-// Exclusive prefix of the tile counts of the level's large segments (one CTA).
-// Also resets the level's counters (tile counter, rows moved, next-level
-// count) so that no separate memsets are needed.
+// Exclusive prefix of the tile (or chunk) counts of the listed segments (one CTA).
+// With long_rows, the super rows of the segments of more than kSuper tiles are
+// listed there (*nlong of them).
 __device__ __forceinline__ void tile_prefix_body(const LargeSeg *segs, uint32_t nseg, uint32_t *tile_prefix,
-                                                 uint32_t tile_rows, bool chunks = false)
+                                                 uint32_t tile_rows, uint2 *long_rows = nullptr,
+                                                 uint32_t *nlong = nullptr)
 {
     __shared__ uint32_t warp_sums[32];
     __shared__ uint32_t carry;
@@ -364,9 +365,11 @@ __device__ __forceinline__ void tile_prefix_body(const LargeSeg *segs, uint32_t 
     __syncthreads();
     for (uint32_t base = 0; base < nseg; base += blockDim.x) {
         const uint32_t s = base + threadIdx.x;
-        const uint32_t c = s >= nseg ? 0u
-                           : chunks  ? seg_chunks(segs[s].len, tile_rows)
-                                     : (segs[s].len + tile_rows - 1) / tile_rows;
+        const uint32_t c = s >= nseg ? 0u : seg_chunks(segs[s].len, tile_rows);
+        if (long_rows && c > kSuper) {
+            const uint32_t k = (c - 1) / kSuper + 1, at = atomicAdd(nlong, k);
+            for (uint32_t i = 0; i < k; ++i) long_rows[at + i] = make_uint2(s, i);
+        }
         uint32_t incl = c;
         for (int o = 1; o < 32; o <<= 1) {
             uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
@@ -401,10 +404,10 @@ __global__ void __launch_bounds__(1024) tile_prefix_kernel(const LargeSeg *segs,
     tile_prefix_body(segs, *d_nseg, tile_prefix, tile_rows);
 }
 
-// First launch of an MSD level: tile prefix of the level's large segments,
+// First launch of an MSD level: chunk prefix of the level's large segments,
 // resets of the level's counters, and (device-side levels) the level index
 // advanced for the level's other launches.
-__global__ void __launch_bounds__(1024) level_prefix_kernel(LevelRefs r, uint32_t *tile_prefix, uint32_t tile_rows)
+__global__ void __launch_bounds__(1024) level_prefix_kernel(LevelRefs r)
 {
     kernel_prologue();
     const uint32_t lvl = r.dev_level ? r.ctr[kCtrLevel] : 0u;
@@ -413,26 +416,23 @@ __global__ void __launch_bounds__(1024) level_prefix_kernel(LevelRefs r, uint32_
     __syncthreads();   // every thread has read the level index before it advances
     if (threadIdx.x == 0) {
         r.ctr[kCtrLarge0 + nxt] = 0;
-        r.ctr[kCtrChunks0 + nxt] = 0;
         r.ctr[kCtrMsdTile] = 0;
         r.ctr[kCtrMoved] = 0;
+        r.ctr[kCtrWork] = 0;
+        r.ctr[kCtrLong] = 0;
         if (r.dev_level) r.ctr[kCtrLevel] = lvl + 1;
     }
-    const LargeSeg *segs = cur ? r.large[1] : r.large[0];
-    tile_prefix_body(segs, nseg, tile_prefix, tile_rows);
-    if (r.chunk_prefix) {
-        tile_prefix_body(segs, nseg, r.chunk_prefix, tile_rows, true);
-        if (lvl == 0 && !r.hist0_ready) {
-            // level 0's histogram rows start at zero (a level's scatter zeroes
-            // the next level's rows)
-            __syncthreads();
-            const uint64_t words = (uint64_t)r.chunk_prefix[nseg] * (kRadix / 4);
-            uint4 *h = reinterpret_cast<uint4 *>(cur ? r.hist[1] : r.hist[0]);
-            for (uint64_t i = threadIdx.x; i < words; i += blockDim.x) h[i] = make_uint4(0, 0, 0, 0);
-        }
+    __syncthreads();
+    tile_prefix_body(cur ? r.large[1] : r.large[0], nseg, r.chunk_prefix, r.chunk_rows, r.long_rows,
+                     &r.ctr[kCtrLong]);
+    if (lvl == 0 && !r.top_hist) {
+        // level 0's super rows start at zero (a level's scatter zeroes the next level's)
+        __syncthreads();
+        const uint64_t words = nseg ? (uint64_t)(super_row(r.chunk_prefix[nseg], nseg) + 1) * (kRadix / 4) : 0;
+        uint4 *h = reinterpret_cast<uint4 *>(r.super[0]);
+        for (uint64_t i = threadIdx.x; i < words; i += blockDim.x) h[i] = make_uint4(0, 0, 0, 0);
     }
 }
-
 
 // The segment of tile t (tile_prefix[s] <= t < tile_prefix[s + 1]), found by
 // a whole warp (t the same in every lane): each round the 32 lanes probe 32
@@ -455,236 +455,215 @@ __device__ __forceinline__ uint32_t find_segment_warp(const uint32_t *tile_prefi
     return lo;
 }
 
-// Top-digit histogram of every large segment.  A block takes a contiguous run
-// of tiles; each thread issues all of a tile's loads before counting (up to 16
-// in flight), and each warp counts into its own shared sub-histogram so that
-// skewed digits do not serialize the whole block on one counter.
+// Top-digit histogram of every chunk, added to its super row as well.  A CTA
+// takes a contiguous run of chunks and reads whole ones, so a chunk's row is
+// stored, not added to.  Each thread issues all of a tile's loads before
+// counting (up to 16 in flight), and each warp counts into its own shared
+// sub-histogram so that skewed digits do not serialize the whole block on one
+// counter.  Two sets of them alternate by chunk: one is written out while the
+// next chunk's loads are in flight, one barrier a chunk.
 template <typename K>
-__global__ void __launch_bounds__(kNtM, kHistCtas) msd_hist_kernel(Bufs<K> b, LevelRefs r, const uint32_t *tile_prefix,
-                                                        uint32_t tile_rows)
+__global__ void __launch_bounds__(kNtM, kHistCtas) msd_hist_kernel(Bufs<K> b, LevelRefs r)
 {
     kernel_prologue();
     constexpr int NW = kNtM / 32;
-    constexpr int MAXJ = 16;   // tile_rows <= 16 * kNtM
-    __shared__ uint32_t sh[NW][kRadix];
+    constexpr int MAXJ = 16;
+    __shared__ uint32_t sh[2][NW][kRadix];
     const uint32_t lvl = running_level(r);
-    if (lvl == 0 && r.hist0_ready) return;
+    if (lvl == 0 && r.top_hist) return;
     const uint32_t cur = lvl & 1u;
     const LargeSeg *segs = (cur ? r.large[1] : r.large[0]);
-    uint32_t *hist = (cur ? r.hist[1] : r.hist[0]);
+    uint32_t *super = (cur ? r.super[1] : r.super[0]);
     const uint32_t nseg = r.ctr[kCtrLarge0 + cur];
     if (nseg == 0) return;
-    const uint32_t T = tile_prefix[nseg];
-    const int warp = threadIdx.x >> 5;
-    // a contiguous run of tiles per block; the per-warp counts are added to
-    // the segment's histogram when the run moves to the next segment (every
-    // large segment has at least one tile) and at its end
-    const uint32_t per = (T + gridDim.x - 1) / gridDim.x;
-    const uint32_t t0 = blockIdx.x * per;
-    const uint32_t t1 = min(T, t0 + per);
-    if (t0 >= T) return;
-    for (int d = threadIdx.x; d < NW * kRadix; d += blockDim.x) (&sh[0][0])[d] = 0;
-    uint32_t s = find_segment_warp(tile_prefix, nseg, t0);
+    const uint32_t C = r.chunk_prefix[nseg];
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t per = (C + gridDim.x - 1) / gridDim.x;
+    const uint32_t q0 = blockIdx.x * per, q1 = min(C, q0 + per);
+    if (q0 >= C) return;
+    for (int d = threadIdx.x; d < 2 * NW * kRadix; d += blockDim.x) (&sh[0][0][0])[d] = 0;
+    uint32_t s = find_segment_warp(r.chunk_prefix, nseg, q0);
     LargeSeg sg = segs[s];
-    uint32_t sfirst = tile_prefix[s], snext = tile_prefix[s + 1];
-    // the histogram row of the tiles counted so far: the segment's, or its
-    // chunk's when the level cuts segments into chunks
-    auto row_of = [&](uint32_t seg, uint32_t k) -> uint32_t {
-        return r.chunk_prefix ? r.chunk_prefix[seg] + k / kChunkTiles : seg;
+    uint32_t sfirst = r.chunk_prefix[s], snext = r.chunk_prefix[s + 1];
+    uint32_t prow = 0, psup = 0;   // the chunk to write out
+    // up to MAXJ rows a thread of [beg, end) of the segment; the source switch
+    // is taken once a tile
+    auto load_tile = [&](K (&key)[MAXJ], uint32_t beg, uint32_t end) {
+        if (sg.src == kSrcExt && b.ext_order) {
+            const uint32_t *os = b.ext_order + sg.start;
+            uint32_t v[MAXJ];
+#pragma unroll
+            for (int j = 0; j < MAXJ; ++j) {
+                const uint32_t i = beg + threadIdx.x + j * kNtM;
+                v[j] = i < end ? os[i] : 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < MAXJ; ++j) {
+                const uint32_t i = beg + threadIdx.x + j * kNtM;
+                key[j] = i < end ? b.ext_bank[v[j]] : K(0);
+            }
+        } else {
+            const K *ks = (sg.src == kSrcExt ? b.ext_bank : sg.src == kSrcBuf1 ? b.k1 : b.k0) + sg.start;
+#pragma unroll
+            for (int j = 0; j < MAXJ; ++j) {
+                const uint32_t i = beg + threadIdx.x + j * kNtM;
+                key[j] = i < end ? ks[i] : K(0);
+            }
+        }
     };
-    uint32_t row = row_of(s, t0 - sfirst);
-    auto flush = [&]() {
-        __syncthreads();
-        for (int d = threadIdx.x; d < kRadix; d += blockDim.x) {
+    __syncthreads();
+    for (uint32_t q = q0; q <= q1; ++q) {
+        const uint32_t set = (q - q0) & 1u;
+        K key[MAXJ];
+        uint32_t beg = 0, end = 0, lo = 0, width = 0;
+        if (q < q1) {
+            if (q >= snext) {   // every large segment has a chunk: the next chunk starts the next segment
+                ++s;
+                sg = segs[s];
+                sfirst = snext;
+                snext = r.chunk_prefix[s + 1];
+            }
+            width = sg.shift < (uint32_t)kRadixBits ? sg.shift : (uint32_t)kRadixBits;
+            lo = sg.shift - width;
+            const uint32_t o = (q - sfirst) * r.chunk_rows;
+            beg = o;
+            end = o + min(r.chunk_rows, sg.len - o);
+            load_tile(key, beg, end);
+        }
+        if (q > q0) {
+            // the chunk before, counted in the other set
+            const uint32_t d = threadIdx.x;
             uint32_t c = 0;
 #pragma unroll
             for (int w = 0; w < NW; ++w) {
-                c += sh[w][d];
-                sh[w][d] = 0;
+                c += sh[set ^ 1u][w][d];
+                sh[set ^ 1u][w][d] = 0;
             }
-            if (c) atomicAdd(&hist[(uint64_t)row * kRadix + d], c);
+            r.hist[(uint64_t)prow * kRadix + d] = c;
+            if (c) atomicAdd(&super[(uint64_t)psup * kRadix + d], c);
         }
+        if (q == q1) break;
+        for (;;) {
+#pragma unroll
+            for (int j = 0; j < MAXJ; ++j) {
+                const uint32_t i = beg + threadIdx.x + j * kNtM;
+                if (i < end) atomicAdd(&sh[set][warp][digit_of(key[j], lo, width)], 1u);
+            }
+            beg += MAXJ * kNtM;
+            if (beg >= end) break;
+            load_tile(key, beg, end);
+        }
+        prow = q;
+        psup = super_row(sfirst, s) + (q - sfirst) / kSuper;
         __syncthreads();
-    };
-    __syncthreads();
-    for (uint32_t t = t0; t < t1; ++t) {
-        if (t >= snext) {   // every large segment has a tile: the next tile starts the next segment
-            ++s;
-            sg = segs[s];
-            sfirst = snext;
-            snext = tile_prefix[s + 1];
-        }
-        const uint32_t k = t - sfirst;
-        const uint32_t trow = row_of(s, k);
-        if (trow != row) {
-            flush();
-            row = trow;
-        }
-        const uint32_t width = sg.shift < (uint32_t)kRadixBits ? sg.shift : (uint32_t)kRadixBits;
-        const uint32_t lo = sg.shift - width;
-        const uint64_t beg = (uint64_t)sg.start + (uint64_t)k * tile_rows;
-        const uint64_t end = min((uint64_t)sg.start + sg.len, beg + tile_rows);
-        K key[MAXJ];
-#pragma unroll
-        for (int j = 0; j < MAXJ; ++j) {
-            const uint64_t i = beg + threadIdx.x + (uint64_t)j * kNtM;
-            if (i < end) key[j] = load_k(b, sg.src, i);
-        }
-#pragma unroll
-        for (int j = 0; j < MAXJ; ++j) {
-            const uint64_t i = beg + threadIdx.x + (uint64_t)j * kNtM;
-            if (i < end) atomicAdd(&sh[warp][digit_of(key[j], lo, width)], 1u);
-        }
     }
-    flush();
 }
 
-// Per large segment: exclusive digit offsets, skip detection, children.
-// With chunks, a segment's digit counts are the sums of its chunks' rows, and
-// each chunk's row becomes its digit bases: the segment's offset of the digit
-// plus the digit's rows in the segment's earlier chunks.  kPlanThreads threads
-// per segment: kPlanThreads / kRadix of them per digit, each summing (then
-// rewriting) a contiguous share of the chunk rows with kPlanLoads loads in
-// flight, so that a segment of a hundred chunks costs a few round trips.
-// (1024 threads per segment walk long segments faster, but four times fewer
-// segments are planned at once: slower in all.)
+// Per large segment: its digit totals (the sum of its super rows), exclusive
+// digit offsets, skip detection, children, its chunks' digit bases (the
+// segment's start and offset of the digit plus the digit's rows in the earlier
+// chunks), and its chunks listed for the scatter.  A segment of up to kSuper
+// chunks is one CTA's work; of a longer one (a round's first level; skew) a CTA
+// does each super row's chunks.  A thread per digit, kPlanLoads loads in flight.
 constexpr int kPlanThreads = 256;
 constexpr int kPlanLoads = 16;
-constexpr int kPlanHelpers = 8;   // CTAs writing level 0's chunk bases beside the segment's CTA
-static_assert(kRadix % kPlanHelpers == 0 && kPlanThreads % (kRadix / kPlanHelpers) == 0 &&
-              kPlanThreads / (kRadix / kPlanHelpers) <= 32, "plan helper layout");
+static_assert(kPlanThreads == kRadix, "a thread per digit");
 
-__global__ void __launch_bounds__(kPlanThreads) msd_plan_kernel(LevelRefs r, Lists lists, bool emit_children = true,
-                                                                uint32_t tile_rows = 0)
+__global__ void __launch_bounds__(kPlanThreads) msd_plan_kernel(LevelRefs r, Lists lists, bool emit_children = true)
 {
     kernel_prologue();
-    constexpr int NQ = kPlanThreads / kRadix;   // threads per digit
     __shared__ uint32_t cnt[kRadix];
-    __shared__ uint32_t part[NQ][kRadix];
     __shared__ uint32_t tmp[kPlanThreads / 32 + 1];
-    __shared__ uint32_t s_skip;
+    __shared__ uint32_t s_skip, s_work;
     const uint32_t lvl = running_level(r);
     const uint32_t cur = lvl & 1u, nxt = cur ^ 1u;
     LargeSeg *segs = (cur ? r.large[1] : r.large[0]);
-    uint32_t *hist = (cur ? r.hist[1] : r.hist[0]);
-    // the counts: this level's rows, or at level 0 the stitch's
-    const uint32_t *counts = (lvl == 0 && r.hist0_ready && r.top_hist) ? r.top_hist : hist;
-    uint32_t *ctr = r.ctr;
-    const int next_large_ctr = kCtrLarge0 + (int)nxt;
     LargeSeg *large_next = (nxt ? r.large[1] : r.large[0]);
-    const uint32_t nseg = ctr[kCtrLarge0 + cur];
-    const uint32_t d = threadIdx.x % kRadix;
-    const uint32_t q4 = threadIdx.x / kRadix;
-    // Level 0 counted by the stitch: one segment with its totals in the last
-    // row.  CTA 0 plans the segment; CTAs 1..kPlanHelpers write the chunk
-    // bases, each for kRadix / kPlanHelpers digits with kPlanThreads /
-    // (kRadix / kPlanHelpers) threads per digit, each over a share of the rows
-    // (a scan across the digit's threads joins the shares).
-    const bool split0 = counts == r.top_hist && r.chunk_prefix != nullptr;
-    if (split0 && blockIdx.x >= 1 && blockIdx.x <= (unsigned)kPlanHelpers && nseg == 1) {
-        constexpr uint32_t DPB = kRadix / kPlanHelpers;        // digits per helper CTA
-        constexpr uint32_t TPD = kPlanThreads / DPB;           // threads per digit (a power of two <= 32)
-        const uint32_t nrows = r.chunk_prefix[1];
-        cnt[d] = q4 == 0 ? counts[(uint64_t)nrows * kRadix + d] : 0u;
-        uint32_t total;
-        block_exclusive_scan_radix<kPlanThreads>(cnt, tmp, &total);
-        const uint32_t dd = (blockIdx.x - 1) * DPB + threadIdx.x / TPD;
-        const uint32_t sub = threadIdx.x % TPD;
-        const uint32_t per = (nrows + TPD - 1) / TPD;
-        const uint32_t qa = min(nrows, sub * per), qb = min(nrows, qa + per);
+    const uint32_t nseg = r.ctr[kCtrLarge0 + cur];
+    if (nseg == 0) return;
+    const bool top = lvl == 0 && r.top_hist;   // one segment, counted by the stitch
+    const uint32_t *counts = top ? r.top_hist : r.hist;
+    const uint32_t *super = top ? r.top_hist + (uint64_t)r.chunk_prefix[1] * kRadix
+                                : (cur ? r.super[1] : r.super[0]);
+    const uint32_t d = threadIdx.x;
+    // Sum of digit d over rows [q, q1) of an array of rows.
+    auto sum_rows = [&](const uint32_t *rows, uint32_t q, uint32_t q1) -> uint32_t {
         uint32_t c = 0;
-        for (uint32_t q = qa; q < qb; q += kPlanLoads) {
+        for (; q < q1; q += kPlanLoads) {
             uint32_t v[kPlanLoads];
 #pragma unroll
-            for (int j = 0; j < kPlanLoads; ++j) v[j] = q + j < qb ? counts[(uint64_t)(q + j) * kRadix + dd] : 0u;
+            for (int j = 0; j < kPlanLoads; ++j) v[j] = q + j < q1 ? rows[(uint64_t)(q + j) * kRadix + d] : 0u;
 #pragma unroll
             for (int j = 0; j < kPlanLoads; ++j) c += v[j];
         }
-        // exclusive scan of the shares across the digit's TPD lanes
-        uint32_t incl = c;
-#pragma unroll
-        for (uint32_t o = 1; o < TPD; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o, TPD);
-            if (sub >= o) incl += y;
-        }
-        uint32_t run = cnt[dd] + incl - c;
-        for (uint32_t q = qa; q < qb; q += kPlanLoads) {
+        return c;
+    };
+    // Exclusive digit offsets into cnt from the digit totals; true when one
+    // digit holds every row (the pass is the identity).
+    auto offsets = [&](uint32_t t, uint32_t len) -> bool {
+        if (d == 0) s_skip = 0;
+        __syncthreads();
+        cnt[d] = t;
+        if (t == len) s_skip = 1;
+        uint32_t total;
+        block_exclusive_scan_radix<kPlanThreads>(cnt, tmp, &total);
+        return s_skip != 0;
+    };
+    // Chunk rows [q, q1) become bases, running on from `run`.
+    auto write_bases = [&](uint32_t q, uint32_t q1, uint32_t run) {
+        for (; q < q1; q += kPlanLoads) {
             uint32_t v[kPlanLoads];
 #pragma unroll
-            for (int j = 0; j < kPlanLoads; ++j) v[j] = q + j < qb ? counts[(uint64_t)(q + j) * kRadix + dd] : 0u;
+            for (int j = 0; j < kPlanLoads; ++j) v[j] = q + j < q1 ? counts[(uint64_t)(q + j) * kRadix + d] : 0u;
 #pragma unroll
             for (int j = 0; j < kPlanLoads; ++j) {
-                if (q + j < qb) hist[(uint64_t)(q + j) * kRadix + dd] = run;
+                if (q + j < q1) r.hist[(uint64_t)(q + j) * kRadix + d] = run;
                 run += v[j];
             }
         }
-        return;
+    };
+    const uint32_t nitems = r.ctr[kCtrLong];
+    for (uint32_t i = gridDim.x - 1 - blockIdx.x; i < nitems; i += gridDim.x) {
+        const uint2 it = r.long_rows[i];
+        const LargeSeg sg = segs[it.x];
+        const uint32_t r0 = r.chunk_prefix[it.x], r1 = r.chunk_prefix[it.x + 1];
+        const uint32_t s0 = top ? 0u : super_row(r0, it.x), ns = (r1 - r0 - 1) / kSuper + 1;
+        const uint32_t before = sum_rows(super, s0, s0 + it.y);
+        const bool skip = offsets(before + sum_rows(super, s0 + it.y, s0 + ns), sg.len);
+        const uint32_t q = r0 + it.y * kSuper;
+        if (!skip) write_bases(q, min(r1, q + kSuper), sg.start + cnt[d] + before);
+        __syncthreads();
     }
     for (uint32_t s = blockIdx.x; s < nseg; s += gridDim.x) {
         const LargeSeg sg = segs[s];
-        const uint32_t r0 = r.chunk_prefix ? r.chunk_prefix[s] : s;
-        const uint32_t r1 = r.chunk_prefix ? r.chunk_prefix[s + 1] : s + 1;
-        // this thread's share of the rows
-        const uint32_t per = (r1 - r0 + NQ - 1) / NQ;
-        const uint32_t qa = min(r1, r0 + q4 * per), qb = min(r1, qa + per);
-        uint32_t c = 0;
-        if (counts == r.top_hist) {
-            // the stitch's rows end with the (one) segment's total
-            if (q4 == 0) c = counts[(uint64_t)r1 * kRadix + d];
-        } else {
-            for (uint32_t q = qa; q < qb; q += kPlanLoads) {
-                uint32_t v[kPlanLoads];
-#pragma unroll
-                for (int j = 0; j < kPlanLoads; ++j) v[j] = q + j < qb ? counts[(uint64_t)(q + j) * kRadix + d] : 0u;
-#pragma unroll
-                for (int j = 0; j < kPlanLoads; ++j) c += v[j];
-            }
-        }
-        part[q4][d] = c;
-        if (threadIdx.x == 0) s_skip = 0;
-        __syncthreads();
-        uint32_t tot = 0;
-        if (q4 == 0) {
-#pragma unroll
-            for (int j = 0; j < NQ; ++j) tot += part[j][d];
-            cnt[d] = tot;
-            if (tot == sg.len) s_skip = 1;   // every row has this digit: the pass is the identity
-        }
-        uint32_t total;
-        block_exclusive_scan_radix<kPlanThreads>(cnt, tmp, &total);
+        const uint32_t r0 = r.chunk_prefix[s], r1 = r.chunk_prefix[s + 1];
+        const uint32_t s0 = top ? 0u : super_row(r0, s);
+        const uint32_t tot = sum_rows(super, s0, s0 + (r1 - r0 - 1) / kSuper + 1);
+        const bool skip = offsets(tot, sg.len);
         const uint32_t off = cnt[d];
-        // this share's first base: the digit's offset plus the earlier shares' rows
-        uint32_t run = off;
-        for (uint32_t j = 0; j < q4; ++j) run += part[j][d];
-        // (with split0 and one segment the helper CTAs write the bases)
-        for (uint32_t q = qa; q < (split0 && nseg == 1 ? qa : qb); q += kPlanLoads) {
-            uint32_t v[kPlanLoads];
-#pragma unroll
-            for (int j = 0; j < kPlanLoads; ++j) v[j] = q + j < qb ? counts[(uint64_t)(q + j) * kRadix + d] : 0u;
-#pragma unroll
-            for (int j = 0; j < kPlanLoads; ++j) {
-                if (q + j < qb) hist[(uint64_t)(q + j) * kRadix + d] = run;
-                run += v[j];
+        if (d == 0) {
+            if (skip) {
+                segs[s].src = sg.src | kSkipBit;
+            } else {
+                s_work = atomicAdd(&r.ctr[kCtrWork], r1 - r0);
+                atomicAdd(&r.ctr[kCtrMoved], sg.len);
             }
         }
-        const bool skip = s_skip != 0;
-        const uint32_t width = sg.shift < (uint32_t)kRadixBits ? sg.shift : (uint32_t)kRadixBits;
-        const uint32_t child_shift = sg.shift - width;
-        const uint32_t child_src = skip ? sg.src : (sg.src == kSrcBuf1 ? kSrcBuf0 : kSrcBuf1);
-        if (q4 == 0 && emit_children && tot > 0) {
-            // (the next level's histogram rows are zeroed by the scatter grid)
-            const int which = route_segment(sg.start + off, tot, child_shift, child_src, ctr, next_large_ctr,
-                                            large_next, lists, nullptr);
-            if (r.chunk_prefix) {
-                // the large children's chunks, one atomic per warp
-                const uint32_t mask = __activemask();
-                const uint32_t add = __reduce_add_sync(mask, which == next_large_ctr ? seg_chunks(tot, tile_rows)
-                                                                                     : 0u);
-                if ((int)lane_id() == __ffs(mask) - 1 && add) atomicAdd(&ctr[kCtrChunks0 + nxt], add);
+        if (!skip && r1 - r0 <= kSuper) write_bases(r0, r1, sg.start + off);
+        __syncthreads();
+        if (!skip) {
+            for (uint32_t q = r0 + d; q < r1; q += kPlanThreads) {
+                const uint32_t o = (q - r0) * r.chunk_rows;
+                r.work[s_work + (q - r0)] = Chunk{sg.start + o, min(r.chunk_rows, sg.len - o), q,
+                                                  sg.shift | (sg.src << 8)};
             }
         }
-        if (threadIdx.x == 0 && skip) segs[s].src = sg.src | kSkipBit;
-        if (threadIdx.x == 0 && !skip) atomicAdd(&ctr[kCtrMoved], sg.len);
+        if (emit_children && tot > 0) {
+            const uint32_t width = sg.shift < (uint32_t)kRadixBits ? sg.shift : (uint32_t)kRadixBits;
+            const uint32_t child_src = skip ? sg.src : (sg.src == kSrcBuf1 ? kSrcBuf0 : kSrcBuf1);
+            route_segment(sg.start + off, tot, sg.shift - width, child_src, r.ctr, kCtrLarge0 + (int)nxt, large_next,
+                          lists);
+        }
         __syncthreads();
     }
 }
@@ -694,22 +673,34 @@ constexpr int msd_ctas_per_sm(int it) { return it >= 16 ? kMsdCtas16 : 4; }
 
 template <typename K, int IT>
 struct MsdSmem {
-    uint32_t whist[kNtM / 32][kRadix];
-    uint32_t total[kRadix];
+    uint32_t whist[kNtM / 32][kRadix];   // per warp and digit: rows so far, then where they go in the tile
     uint32_t doff[kRadix];       // tile-local exclusive digit offsets
     uint32_t gdst[kRadix];       // global destination base per digit (mod 2^32; rows < 2^32)
-    uint32_t tmp[kNtM / 32 + 1];
-    uint32_t tile, seg;
+    Chunk next;
+    uint32_t tmp[kNtM / 32 + 4];
     K keys[kNtM * IT];
     uint32_t vals[kNtM * IT];
     static_assert(kNtM * IT >= (kNtM / 32) * kRadix, "the peer words of kRankOr fit in vals");
+    static_assert(kNtM == kRadix, "a thread per digit");
 };
 
+// Moves the level's chunks: a CTA claims a chunk and takes its tiles in order.
+// Per tile: rank (stable, by warp-level multi-split), digit offsets, rows staged
+// in digit order, written out in runs.  As soon as a tile is staged its
+// registers take the loads of the next one (of this chunk, or of the next
+// chunk, claimed while this one's first tile was ranked), which so run during
+// the write-out.
+// Bound: the shared-memory pipe (83% busy; about 50 wavefronts per 32 rows: the
+// peer word's OR, load and clear, the counter's load and store, the rank's
+// base, staging both arrays and reading them back).  One level over 16.8M rows
+// of 8-byte keys: 108 us, 24 bytes a row at 3.7 TB/s; 130 us when every tile
+// also waited for its predecessors' digit counts (decoupled look-back).
+// Counters and peer bits in one 64-bit word (fewer accesses, but 64-bit ones):
+// 131 us; ballots instead of the OR: 117; match.any: 156.
 template <typename K, int RANK, int IT>
 __global__ void __launch_bounds__(kNtM, msd_ctas_per_sm(IT)) msd_scatter_kernel(Bufs<K> b, LevelRefs r,
-                                                           const uint32_t *tile_prefix, unsigned long long *lookback,
-                                                           uint32_t epoch_base, int *status,
-                                                           cudaGraphConditionalHandle more, uint32_t levels)
+                                                                                cudaGraphConditionalHandle more,
+                                                                                uint32_t levels)
 {
     kernel_prologue();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -717,65 +708,54 @@ __global__ void __launch_bounds__(kNtM, msd_ctas_per_sm(IT)) msd_scatter_kernel(
     constexpr uint32_t kTileM = kNtM * IT;
     const uint32_t lvl = running_level(r);
     const uint32_t cur = lvl & 1u;
-    const LargeSeg *segs = (cur ? r.large[1] : r.large[0]);
-    const uint32_t *offs = (cur ? r.hist[1] : r.hist[0]);
-    uint32_t *tile_counter = &r.ctr[kCtrMsdTile];
-    const uint32_t epoch = epoch_base + lvl;
-    const uint32_t nseg = r.ctr[kCtrLarge0 + cur];
     // Inside a graph, the level loop goes on while the next level has large
     // segments (msd_plan has counted them before this launch).
     const uint32_t nnext = r.ctr[kCtrLarge0 + (cur ^ 1u)];
     if (more && blockIdx.x == 0 && threadIdx.x == 0)
         cudaGraphSetConditional(more, (nnext > 0 && lvl + 1 < levels) ? 1u : 0u);
     {
-        // the histogram rows of the next level's large segments (or of their
-        // chunks, counted by this level's plan) start at zero (the rows held
-        // this level's predecessor's offsets, which nothing reads any more)
-        uint4 *h = reinterpret_cast<uint4 *>(cur ? r.hist[0] : r.hist[1]);
-        const uint32_t rows_next = r.chunk_prefix ? r.ctr[kCtrChunks0 + (cur ^ 1u)] : nnext;
-        const uint64_t words = (uint64_t)rows_next * (kRadix / 4);
+        // the next level's super rows start at zero (they held the previous
+        // level's, which nothing reads any more)
+        uint4 *h = reinterpret_cast<uint4 *>(cur ? r.super[0] : r.super[1]);
+        const uint64_t words = nnext ? super_rows_max(r.max_chunks, nnext) * (kRadix / 4) : 0;
         for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < words;
              i += (uint64_t)gridDim.x * blockDim.x)
             h[i] = make_uint4(0, 0, 0, 0);
     }
-    if (nseg == 0) return;
-    const uint32_t T = tile_prefix[nseg];
+    const uint32_t C = r.ctr[kCtrWork];
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    for (;;) {
-        if (threadIdx.x == 0) sm.tile = atomicAdd(tile_counter, 1u);
-        __syncthreads();
-        const uint32_t t = sm.tile;
-        if (t >= T) break;
-        const uint32_t s = find_segment_warp(tile_prefix, nseg, t);
-        const LargeSeg sg = segs[s];
-        if (sg.src & kSkipBit) {
-            __syncthreads();
-            continue;
-        }
-        const uint32_t k = t - tile_prefix[s];
-        // the tile's histogram row and its place in its look-back chain
-        const uint32_t row = r.chunk_prefix ? r.chunk_prefix[s] + k / kChunkTiles : s;
-        const uint32_t kc = r.chunk_prefix ? k % kChunkTiles : k;
-        const uint32_t width = sg.shift < (uint32_t)kRadixBits ? sg.shift : (uint32_t)kRadixBits;
-        const uint32_t lo = sg.shift - width;
-        const uint64_t tbeg = (uint64_t)sg.start + (uint64_t)k * kTileM;
-        const uint64_t send = (uint64_t)sg.start + sg.len;
-        const uint32_t cnt = (uint32_t)min((uint64_t)kTileM, send - tbeg);
+    const uint32_t wbase = warp * (IT * 32);
+    // chunk number c of the list, or an empty one past its end
+    auto chunk_at = [&](uint32_t c) -> Chunk { return c < C ? r.work[c] : Chunk{0, 0, 0, 0}; };
+    if (threadIdx.x == 0) sm.next = chunk_at(atomicAdd(&r.ctr[kCtrMsdTile], 1u));
+    __syncthreads();
+    Chunk ck = sm.next;
+    K key[IT];
+    uint32_t val[IT];
+    uint32_t gbase = 0;   // this thread's digit: where the chunk's next row of it goes
+    if (ck.len) {
+        load_rows<K, IT>(b, ck.info >> 8, ck.start, min(ck.len, kTileM), IT, wbase, key, val);
+        gbase = r.hist[(uint64_t)ck.row * kRadix + threadIdx.x];
+    }
+    bool first = true;   // the chunk's first tile
+    while (ck.len) {
+        const uint32_t src = ck.info >> 8, shift = ck.info & 0xFFu;
+        const uint32_t cnt = min(ck.len, kTileM);
+        const uint32_t width = shift < (uint32_t)kRadixBits ? shift : (uint32_t)kRadixBits;
+        const uint32_t lo = shift - width;
+        uint32_t claimed = 0;
+        if (first && threadIdx.x == 0) claimed = atomicAdd(&r.ctr[kCtrMsdTile], 1u);
         // kRankOr's per-warp peer words live in the vals staging area, which
         // is free until the ranks are known
         uint32_t *peerw = &sm.vals[warp * kRadix];
-        for (int d = lane; d < kRadix; d += 32) {
-            sm.whist[warp][d] = 0;
-            if constexpr (RANK == kRankOr) peerw[d] = 0;
+#pragma unroll
+        for (int d = lane; d < kRadix / 4; d += 32) {
+            reinterpret_cast<uint4 *>(sm.whist[warp])[d] = make_uint4(0, 0, 0, 0);
+            if constexpr (RANK == kRankOr) reinterpret_cast<uint4 *>(peerw)[d] = make_uint4(0, 0, 0, 0);
         }
         __syncwarp();
-
-        K key[IT];
-        uint32_t val[IT];
         uint32_t rd[IT];   // rank in the warp (low 16 bits) | digit << 16
-        const uint32_t wbase = warp * (IT * 32);
-        load_rows<K, IT>(b, sg.src, (uint32_t)tbeg, cnt, IT, wbase, key, val);
         if (cnt == kTileM && width == (uint32_t)kRadixBits) {
             // a whole tile and a whole digit (the common case): no lane checks
 #pragma unroll
@@ -797,43 +777,28 @@ __global__ void __launch_bounds__(kNtM, msd_ctas_per_sm(IT)) msd_scatter_kernel(
                     rd[j] = wlms_rank<RANK>(d, p < cnt, sm.whist[warp], width) | (d << 16);
             }
         }
+        if (first && threadIdx.x == 0) sm.next = chunk_at(claimed);
         __syncthreads();
-        // per digit: exclusive over warps, tile total
-        for (int d = threadIdx.x; d < kRadix; d += kNtM) {
-            uint32_t run = 0;
+        // this thread's digit: its rows per warp, tile total
+        uint32_t wc[kNtM / 32], total = 0;
 #pragma unroll
-            for (int w = 0; w < kNtM / 32; ++w) {
-                const uint32_t c = sm.whist[w][d];
-                sm.whist[w][d] = run;
-                run += c;
-            }
-            sm.total[d] = run;
-            sm.doff[d] = run;
-            unsigned long long *mine = &lookback[(uint64_t)t * kRadix + d];
-            st_volatile_u64(mine, lb_word(epoch, kc == 0 ? kFlagInclusive : kFlagAggregate, run));
+        for (int w = 0; w < kNtM / 32; ++w) {
+            wc[w] = sm.whist[w][threadIdx.x];
+            total += wc[w];
         }
+        sm.doff[threadIdx.x] = total;
         __syncthreads();
         uint32_t tot;
         block_exclusive_scan_radix<kNtM>(sm.doff, sm.tmp, &tot);
-        // decoupled look-back along the chunk's tiles
-        for (int d = threadIdx.x; d < kRadix; d += kNtM) {
-            uint32_t excl = 0;
-            if (kc > 0) {
-                int64_t p = (int64_t)t - 1;
-                for (;;) {
-                    const unsigned long long w = lb_wait(&lookback[(uint64_t)p * kRadix + d], epoch, status);
-                    excl += (uint32_t)w;
-                    if (((uint32_t)(w >> 32) & 3u) == kFlagInclusive) break;
-                    --p;
-                }
-                st_volatile_u64(&lookback[(uint64_t)t * kRadix + d],
-                                lb_word(epoch, kFlagInclusive, excl + sm.total[d]));
-            }
-            const uint32_t dof = sm.doff[d];
-            sm.gdst[d] = sg.start + offs[(uint64_t)row * kRadix + d] + excl - dof;   // wraps; + slot is in range
-            // the warps' exclusive counts become tile positions
+        {
+            uint32_t dof = sm.doff[threadIdx.x];
+            sm.gdst[threadIdx.x] = gbase - dof;   // wraps; + slot is in range
+            gbase += total;
 #pragma unroll
-            for (int w = 0; w < kNtM / 32; ++w) sm.whist[w][d] += dof;
+            for (int w = 0; w < kNtM / 32; ++w) {
+                sm.whist[w][threadIdx.x] = dof;
+                dof += wc[w];
+            }
         }
         __syncthreads();
 #pragma unroll
@@ -846,8 +811,17 @@ __global__ void __launch_bounds__(kNtM, msd_ctas_per_sm(IT)) msd_scatter_kernel(
             }
         }
         __syncthreads();
-        K *dk = (sg.src == kSrcBuf1) ? b.k0 : b.k1;
-        uint32_t *dv = (sg.src == kSrcBuf1) ? b.v0 : b.v1;
+        // the next tile's loads: the chunk's, or the first of the next chunk
+        ck.start += cnt;
+        ck.len -= cnt;
+        first = ck.len == 0;
+        if (first) {
+            ck = sm.next;
+            if (ck.len) gbase = r.hist[(uint64_t)ck.row * kRadix + threadIdx.x];
+        }
+        if (ck.len) load_rows<K, IT>(b, ck.info >> 8, ck.start, min(ck.len, kTileM), IT, wbase, key, val);
+        K *dk = (src == kSrcBuf1) ? b.k0 : b.k1;
+        uint32_t *dv = (src == kSrcBuf1) ? b.v0 : b.v1;
         for (uint32_t i = threadIdx.x; i < cnt; i += kNtM) {
             const K kk = sm.keys[i];
             const uint32_t o = sm.gdst[digit_of(kk, lo, width)] + i;
@@ -1518,7 +1492,6 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
 
     // lists (capacities are bounds on disjoint segments of each tier's minimum size)
     const uint32_t local_max = std::max<uint32_t>(kCapA, std::min<uint32_t>(ctx->local_max, kCapLocal));
-    const uint32_t tile_rows = kNtM * IT;
     const uint64_t cap_large = n / (local_max + 1) + 2;
     const uint64_t cap_t = n / 2 + 2, cap_t32 = n / (kCapT + 1) + 2, cap_a = n / (kCapT + 1) + 2;
     const uint64_t cap_a2 = n / (kCapA + 1) + 2, cap_b1 = n / (kCapA2 + 1) + 2;
@@ -1562,32 +1535,45 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
         lists.copy_large = cc.take<LargeSeg>(cap_large);
         lists.local_max = local_max;
     }
-    // histogram rows: one per chunk of kChunkTiles tiles of a large segment
-    // (a segment's chunks <= its tiles / kChunkTiles + 1)
-    const uint64_t max_tiles = n / tile_rows + cap_large + 1;
-    const uint64_t cap_chunks = max_tiles / kChunkTiles + cap_large + 1;
-    uint32_t *hists[2], *tile_prefix, *chunk_prefix;
-    if ((rc = ws_get(ctx, kSlotSegHist, 2 * carve_round(cap_chunks * kRadix * sizeof(uint32_t)), &p))) return rc;
+    // (a segment's chunks <= its rows / chunk_rows + 1)
+    LevelRefs lr{};
+    lr.large[0] = large[0];
+    lr.large[1] = large[1];
+    lr.chunk_rows = msd_chunk_rows(ctx, n);
+    lr.max_chunks = (uint32_t)(n / lr.chunk_rows);
+    const uint64_t cap_chunks = n / lr.chunk_rows + cap_large + 1;
+    const uint64_t cap_super = super_rows_max(cap_chunks, cap_large);
+    const uint64_t cap_long = 2 * (cap_chunks / kSuper) + 2;   // ceil(c / kSuper) <= 2 c / kSuper for c > kSuper
+    const size_t row = kRadix * sizeof(uint32_t);
+    if ((rc = ws_get(ctx, kSlotSegHist,
+                     carve_total({cap_chunks * row, cap_super * row, cap_super * row, cap_chunks * sizeof(Chunk),
+                                  cap_long * sizeof(uint2)}),
+                     &p)))
+        return rc;
     {
         Carver cv(p);
-        hists[0] = cv.take<uint32_t>(cap_chunks * kRadix);
-        hists[1] = cv.take<uint32_t>(cap_chunks * kRadix);
+        lr.hist = cv.take<uint32_t>(cap_chunks * kRadix);
+        lr.super[0] = cv.take<uint32_t>(cap_super * kRadix);
+        lr.super[1] = cv.take<uint32_t>(cap_super * kRadix);
+        lr.work = cv.take<Chunk>(cap_chunks);
+        lr.long_rows = cv.take<uint2>(cap_long);
     }
+    uint32_t *tile_prefix;
     if ((rc = ws_get(ctx, kSlotTilePrefix, carve_total({(cap_large + 1) * sizeof(uint32_t),
                                                         (cap_large + 1) * sizeof(uint32_t)}), &p)))
         return rc;
     {
         Carver cv(p);
         tile_prefix = cv.take<uint32_t>(cap_large + 1);
-        chunk_prefix = cv.take<uint32_t>(cap_large + 1);
+        lr.chunk_prefix = cv.take<uint32_t>(cap_large + 1);
     }
-    unsigned long long *lookback;
-    if ((rc = ws_get(ctx, kSlotLookback, max_tiles * kRadix * sizeof(unsigned long long), &p, true))) return rc;
-    lookback = (unsigned long long *)p;
     uint32_t *ctr;
     if ((rc = ws_get(ctx, kSlotCounters, 4096, &p))) return rc;
     ctr = (uint32_t *)p + 64;   // words 0..63 belong to other kernels
     cudaMemsetAsync(ctr, 0, kCtrWords * sizeof(uint32_t), st);
+    lr.ctr = ctr;
+    lr.dev_level = 1;
+    lr.top_hist = a.seg_start ? nullptr : a.top_hist;
 
     const int sms = ctx->num_sms;
     // classification of the initial segments
@@ -1599,7 +1585,7 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
         if (seg_start && a.nseg_host == 0) grid = (unsigned)sms * 16;
         { LaunchScope ls_(ctx, "classify");
             launch_k(classify_kernel<K>, grid, 256, 0, st, b, seg_start, d_nseg, n, a.key_bits, ctr, large[0], lists,
-                     seg_start ? nullptr : a.top_hist, a.d_key_bits, a.d_in_order,
+                     lr.top_hist, a.d_key_bits, a.d_in_order,
                      a.keys_scratch && a.order_in == a.order_out);
         }
         FMCS_LAUNCH_CHECK("classify");
@@ -1644,26 +1630,21 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
             nlarge = ctx->h_small[16 + kCtrLarge0];
             tiers_known = true;
         }
-        const int hist0_ready = (a.top_hist && !a.seg_start) ? 1 : 0;
-        const LevelRefs lr{{large[0], large[1]}, {hists[0], hists[1]}, ctr, 1, hist0_ready, chunk_prefix,
-                           hist0_ready ? a.top_hist : nullptr};
-        const uint32_t epoch_base = ctx->epoch;
-        ctx->epoch += (uint32_t)levels;
         const unsigned scatter_grid = sms * msd_ctas_per_sm(IT);
         int host_lvl = 0;   // the level being launched, for the eager read-back
         // one level: the same four launches for every level (the level index
         // lives on the device)
         auto level = [&](cudaStream_t s, cudaGraphConditionalHandle more, bool read_back) -> int {
             { LaunchScope ls_(ctx, "tile_prefix");
-                launch_k(level_prefix_kernel, 1, 1024, 0, s, lr, tile_prefix, tile_rows);
+                launch_k(level_prefix_kernel, 1, 1024, 0, s, lr);
             }
-            if (!(hist0_ready && host_lvl == 0 && read_back)) {
+            if (!(lr.top_hist && host_lvl == 0 && read_back)) {
                 // (inside a graph the launch stays and returns at once on level 0)
                 LaunchScope ls_(ctx, "msd_hist");
-                launch_k(msd_hist_kernel<K>, sms * kHistCtas, kNtM, 0, s, b, lr, tile_prefix, tile_rows);
+                launch_k(msd_hist_kernel<K>, sms * kHistCtas, kNtM, 0, s, b, lr);
             }
             { LaunchScope ls_(ctx, "msd_plan");
-                launch_k(msd_plan_kernel, sms * 8, kPlanThreads, 0, s, lr, lists, true, tile_rows);
+                launch_k(msd_plan_kernel, sms * 8, kPlanThreads, 0, s, lr, lists, true);
             }
             if (read_back) {
                 // read the counters (the next level's count, the rows moved,
@@ -1673,9 +1654,8 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
             }
             {
                 LaunchScope ls_(ctx, "msd_scatter");
-                launch_k(msd_scatter_kernel<K, RANK, IT>, scatter_grid, kNtM, msd_smem, s, b, lr, tile_prefix, lookback,
-                                                                                   epoch_base, ctx->d_status, more,
-                                                                                   (uint32_t)levels);
+                launch_k(msd_scatter_kernel<K, RANK, IT>, scatter_grid, kNtM, msd_smem, s, b, lr, more,
+                         (uint32_t)levels);
                 if (read_back) {
                     cudaError_t e = cudaEventSynchronize(ctx->ev_level);
                     if (e != cudaSuccess) return cuda_fail(ctx, e, "sort: level event");
@@ -1844,8 +1824,7 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
 // holding the result is tracked on the device and a final copy puts it in
 // BUF0.
 // ---------------------------------------------------------------------------
-__global__ void lsd_set_pass_kernel(LargeSeg *seg, uint32_t *hist_row, uint32_t *nseg, uint32_t n, uint32_t shift,
-                                    int first)
+__global__ void lsd_set_pass_kernel(LargeSeg *seg, uint32_t *nseg, uint32_t n, uint32_t shift, int first)
 {
     kernel_prologue();
     if (threadIdx.x == 0) {
@@ -1857,7 +1836,6 @@ __global__ void lsd_set_pass_kernel(LargeSeg *seg, uint32_t *hist_row, uint32_t 
         seg[0] = LargeSeg{0, n, shift, src};
         *nseg = 1;
     }
-    for (int d = threadIdx.x; d < kRadix; d += blockDim.x) hist_row[d] = 0;
 }
 
 template <typename K>
@@ -1891,43 +1869,54 @@ int lsd_sort_full_t(fmcs_ctx *ctx, void *keys, uint32_t *vals, uint64_t n, uint3
     LargeSeg *seg;
     if ((rc = ws_get(ctx, kSlotLarge0, sizeof(LargeSeg) * 2, &p))) return rc;
     seg = (LargeSeg *)p;
-    uint32_t *hist, *tile_prefix;
-    if ((rc = ws_get(ctx, kSlotSegHist, 2 * kRadix * sizeof(uint32_t), &p))) return rc;
-    hist = (uint32_t *)p;
-    if ((rc = ws_get(ctx, kSlotTilePrefix, 4 * sizeof(uint32_t), &p))) return rc;
-    tile_prefix = (uint32_t *)p;
-    const uint32_t tile_rows = kNtM * IT;
-    const uint64_t max_tiles = n / tile_rows + 2;
-    unsigned long long *lookback;
-    if ((rc = ws_get(ctx, kSlotLookback, max_tiles * kRadix * sizeof(unsigned long long), &p, true))) return rc;
-    lookback = (unsigned long long *)p;
+    // one segment [0, n), re-set before every pass; level buffers of set 0
+    LevelRefs lr{};
+    lr.large[0] = seg;
+    lr.large[1] = seg + 1;
+    lr.chunk_rows = msd_chunk_rows(ctx, n);
+    lr.max_chunks = (uint32_t)(n / lr.chunk_rows);
+    const uint64_t chunks = (n - 1) / lr.chunk_rows + 1, supers = super_rows_max(chunks, 1);
+    const size_t row = kRadix * sizeof(uint32_t);
+    if ((rc = ws_get(ctx, kSlotSegHist,
+                     carve_total({chunks * row, supers * row, chunks * sizeof(Chunk),
+                                  (chunks / kSuper + 1) * sizeof(uint2)}),
+                     &p)))
+        return rc;
+    {
+        Carver cv(p);
+        lr.hist = cv.take<uint32_t>(chunks * kRadix);
+        lr.super[0] = cv.take<uint32_t>(supers * kRadix);
+        lr.work = cv.take<Chunk>(chunks);
+        lr.long_rows = cv.take<uint2>(chunks / kSuper + 1);
+    }
+    if ((rc = ws_get(ctx, kSlotTilePrefix, 2 * sizeof(uint32_t), &p))) return rc;
+    lr.chunk_prefix = (uint32_t *)p;
     uint32_t *ctr;
     if ((rc = ws_get(ctx, kSlotCounters, 4096, &p))) return rc;
     ctr = (uint32_t *)p + 64;
+    lr.ctr = ctr;
     const size_t msd_smem = sizeof(MsdSmem<K, IT>);
     if ((rc = set_smem(ctx, msd_scatter_kernel<K, RANK, IT>, msd_smem))) return rc;
     const int sms = ctx->num_sms;
     Lists none{};
-    // one segment [0, n), re-set before every pass; level buffers of set 0
-    const LevelRefs lr{{seg, seg + 1}, {hist, hist + kRadix}, ctr, 0, 0};
     int pass = 0;
     for (uint32_t lo = 0; lo < bits; lo += kRadixBits, ++pass) {
         const uint32_t shift = std::min(bits, lo + kRadixBits);
         { LaunchScope ls_(ctx, "lsd_set_pass");
-            launch_k(lsd_set_pass_kernel, 1, 256, 0, st, seg, hist, &ctr[kCtrLarge0], (uint32_t)n, shift, pass == 0);
+            launch_k(lsd_set_pass_kernel, 1, 32, 0, st, seg, &ctr[kCtrLarge0], (uint32_t)n, shift, pass == 0);
         }
         { LaunchScope ls_(ctx, "tile_prefix");
-            launch_k(level_prefix_kernel, 1, 1024, 0, st, lr, tile_prefix, tile_rows);
+            launch_k(level_prefix_kernel, 1, 1024, 0, st, lr);
         }
         { LaunchScope ls_(ctx, "msd_hist");
-            launch_k(msd_hist_kernel<K>, sms * kHistCtas, kNtM, 0, st, b, lr, tile_prefix, tile_rows);
+            launch_k(msd_hist_kernel<K>, sms * kHistCtas, kNtM, 0, st, b, lr);
         }
         { LaunchScope ls_(ctx, "msd_plan");
-            launch_k(msd_plan_kernel, 1, kPlanThreads, 0, st, lr, none, false, tile_rows);
+            launch_k(msd_plan_kernel, sms, kPlanThreads, 0, st, lr, none, false);
         }
         { LaunchScope ls_(ctx, "msd_scatter");
-            launch_k(msd_scatter_kernel<K, RANK, IT>, sms * msd_ctas_per_sm(IT), kNtM, msd_smem, st, 
-                b, lr, tile_prefix, lookback, ctx->epoch++, ctx->d_status, 0, 1u);
+            launch_k(msd_scatter_kernel<K, RANK, IT>, sms * msd_ctas_per_sm(IT), kNtM, msd_smem, st, b, lr,
+                     (cudaGraphConditionalHandle)0, 1u);
         }
         FMCS_LAUNCH_CHECK("lsd pass");
     }
@@ -1941,9 +1930,11 @@ int lsd_sort_full_t(fmcs_ctx *ctx, void *keys, uint32_t *vals, uint64_t n, uint3
 
 }  // namespace
 
-uint32_t msd_chunk_rows(const fmcs_ctx *ctx)
+uint32_t msd_chunk_rows(const fmcs_ctx *ctx, uint64_t n)
 {
-    return kChunkTiles * (uint32_t)kNtM * (ctx->msd_items >= 16 ? 16u : 8u);
+    uint64_t rows = (uint64_t)kNtM * (ctx->msd_items >= 16 ? 16u : 8u);
+    while (rows * 2 * kChunksWanted <= n) rows *= 2;
+    return (uint32_t)rows;
 }
 
 int lsd_sort_full(fmcs_ctx *ctx, void *keys, uint32_t key_bytes, uint32_t *vals, uint64_t n, uint32_t bits)

@@ -91,32 +91,29 @@ __device__ __forceinline__ void store4(B *bank, uint64_t row, bool vec, uint64_t
         if (row + k < n) bank[row + k] = (B)a[k];
 }
 
-// With top_hist the kernel also counts the first radix level's digits, one
-// 256-word row per chunk of 2^chunk_shift rows and, after them, one row for
-// the whole bank; each CTA then takes a contiguous
-// range of block_groups groups of 4 rows (at most one chunk long, so that it
-// meets at most two chunks, counted in two shared histograms).  Without, the
-// groups are spread grid-stride.
+// With top_hist the kernel also counts the first radix level's digits: a CTA
+// takes part_groups groups of 4 rows of one chunk (parts CTAs a chunk) and adds
+// its counts to the chunk's 256-word row and to the chunk's super row after the
+// chunks' rows.  Without, the groups are spread grid-stride.
 template <typename B>
 __global__ void __launch_bounds__(256, 4) stitch_kernel(const __grid_constant__ StitchParams p, B *bank,
                                                      uint64_t n, bool aligned, uint32_t *top_hist,
-                                                     uint32_t hist_lo, uint32_t hist_mask, uint32_t chunk_shift,
-                                                     uint64_t block_groups)
+                                                     uint32_t hist_lo, uint32_t hist_mask, uint64_t chunk_groups,
+                                                     uint32_t part_groups, uint32_t parts)
 {
     kernel_prologue();
-    __shared__ uint32_t sh[2][256];
+    __shared__ uint32_t sh[256];
     const uint64_t groups = (n + 3) / 4;
     // this CTA's groups: [g_begin, g_end), `stride` apart per thread step
     uint64_t g_begin = blockIdx.x * (uint64_t)blockDim.x, g_end = groups;
     uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    uint64_t chunk0 = 0;   // the chunk of the CTA's first row
     if (top_hist) {
-        for (int d = threadIdx.x; d < 2 * 256; d += blockDim.x) (&sh[0][0])[d] = 0;
+        sh[threadIdx.x] = 0;
         __syncthreads();
-        g_begin = blockIdx.x * block_groups;
-        g_end = min(groups, g_begin + block_groups);
+        const uint32_t c = blockIdx.x / parts;
+        g_begin = c * chunk_groups + (uint64_t)(blockIdx.x % parts) * part_groups;
+        g_end = min(min(groups, (c + 1) * chunk_groups), g_begin + part_groups);
         stride = blockDim.x;
-        chunk0 = (g_begin * 4) >> chunk_shift;
     }
     // Each thread takes two groups of 4 rows per step (a stride apart), so
     // that the loads of both are in flight together.
@@ -144,28 +141,20 @@ __global__ void __launch_bounds__(256, 4) stitch_kernel(const __grid_constant__ 
         store4<B>(bank, row0, vec0, n, acc0);
         if (two) store4<B>(bank, row1, vec1, n, acc1);
         if (top_hist) {
-            // a group's 4 rows share a chunk (chunks are at least 4 rows)
-            uint32_t *h0 = sh[(row0 >> chunk_shift) - chunk0];
-            uint32_t *h1 = two ? sh[(row1 >> chunk_shift) - chunk0] : h0;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                if (row0 + k < n) atomicAdd(&h0[(uint32_t)(acc0[k] >> hist_lo) & hist_mask], 1u);
-                if (two && row1 + k < n) atomicAdd(&h1[(uint32_t)(acc1[k] >> hist_lo) & hist_mask], 1u);
+                if (row0 + k < n) atomicAdd(&sh[(uint32_t)(acc0[k] >> hist_lo) & hist_mask], 1u);
+                if (two && row1 + k < n) atomicAdd(&sh[(uint32_t)(acc1[k] >> hist_lo) & hist_mask], 1u);
             }
         }
     }
     if (top_hist) {
         __syncthreads();
-        const uint64_t nchunks = ((n - 1) >> chunk_shift) + 1;
-        for (int i = threadIdx.x; i < 2 * 256; i += blockDim.x) {
-            const uint64_t c = chunk0 + (uint64_t)(i >> 8);
-            const uint32_t v = (&sh[0][0])[i];
-            if (v && c < nchunks) atomicAdd(&top_hist[c * 256 + (i & 255)], v);
-        }
-        // and the whole bank's histogram, the row after the chunks' rows
-        for (int d = threadIdx.x; d < 256; d += blockDim.x) {
-            const uint32_t v = sh[0][d] + sh[1][d];
-            if (v) atomicAdd(&top_hist[nchunks * 256 + d], v);
+        const uint32_t v = sh[threadIdx.x];
+        const uint32_t c = blockIdx.x / parts, chunks = gridDim.x / parts;
+        if (v) {
+            atomicAdd(&top_hist[c * 256ull + threadIdx.x], v);
+            atomicAdd(&top_hist[(chunks + c / kTopSuper) * 256ull + threadIdx.x], v);
         }
     }
 }
@@ -236,42 +225,40 @@ int launch_stitch(fmcs_ctx *ctx, const StitchSlice *sl, int ns, void *bank, uint
     const uint64_t cap = (uint64_t)ctx->num_sms * 8;
     if (blocks > cap) blocks = cap;
     uint32_t hist_lo = 0, hist_mask = 0;
-    uint64_t block_groups = 0;
-    uint32_t chunk_shift = 0;
+    uint64_t chunk_groups = 0;
+    uint32_t part_groups = 0, parts = 1;
     if (top_hist) {
-        if (chunk_rows < 4 || (chunk_rows & (chunk_rows - 1)))
-            return set_error(ctx, FMCS_E_INVAL, "stitch: chunk rows must be a power of two >= 4");
-        chunk_shift = (uint32_t)__builtin_ctz(chunk_rows);
+        if (chunk_rows < 4 || chunk_rows % 4)
+            return set_error(ctx, FMCS_E_INVAL, "stitch: chunk rows must be a multiple of 4");
         const uint32_t width = key_bits < 8u ? key_bits : 8u;
         hist_lo = key_bits - width;
         hist_mask = (1u << width) - 1u;
-        const uint64_t nchunks = (n + chunk_rows - 1) / chunk_rows;
-        cudaMemsetAsync(top_hist, 0, (nchunks + 1) * 256 * sizeof(uint32_t), st);
-        // contiguous ranges of whole 256-group steps, at most one chunk each
-        block_groups = (groups + blocks - 1) / blocks;
-        block_groups = (block_groups + 255) / 256 * 256;
-        const uint64_t chunk_groups = chunk_rows / 4;
-        if (block_groups > chunk_groups) block_groups = chunk_groups;
-        blocks = (groups + block_groups - 1) / block_groups;
+        chunk_groups = chunk_rows / 4;
+        // enough CTAs to fill the GPU, each at least two steps of its threads
+        const uint64_t chunks = (n + chunk_rows - 1) / chunk_rows;
+        parts = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(cap / chunks, chunk_groups / 512));
+        part_groups = (uint32_t)((chunk_groups + parts - 1) / parts);
+        blocks = chunks * parts;
+        cudaMemsetAsync(top_hist, 0, (chunks + (chunks + kTopSuper - 1) / kTopSuper) * 256 * sizeof(uint32_t), st);
     }
     const unsigned grid = (unsigned)blocks;
     LaunchScope ls_(ctx, "stitch");
     switch (bank_bytes) {
     case 1:
         launch_k(stitch_kernel<uint8_t>, grid, 256, 0, st,
-                 p, (uint8_t *)bank, n, aligned, top_hist, hist_lo, hist_mask, chunk_shift, block_groups);
+                 p, (uint8_t *)bank, n, aligned, top_hist, hist_lo, hist_mask, chunk_groups, part_groups, parts);
         break;
     case 2:
         launch_k(stitch_kernel<uint16_t>, grid, 256, 0, st,
-                 p, (uint16_t *)bank, n, aligned, top_hist, hist_lo, hist_mask, chunk_shift, block_groups);
+                 p, (uint16_t *)bank, n, aligned, top_hist, hist_lo, hist_mask, chunk_groups, part_groups, parts);
         break;
     case 4:
         launch_k(stitch_kernel<uint32_t>, grid, 256, 0, st,
-                 p, (uint32_t *)bank, n, aligned, top_hist, hist_lo, hist_mask, chunk_shift, block_groups);
+                 p, (uint32_t *)bank, n, aligned, top_hist, hist_lo, hist_mask, chunk_groups, part_groups, parts);
         break;
     case 8:
         launch_k(stitch_kernel<uint64_t>, grid, 256, 0, st,
-                 p, (uint64_t *)bank, n, aligned, top_hist, hist_lo, hist_mask, chunk_shift, block_groups);
+                 p, (uint64_t *)bank, n, aligned, top_hist, hist_lo, hist_mask, chunk_groups, part_groups, parts);
         break;
     default: return set_error(ctx, FMCS_E_INVAL, "stitch: bank_bytes must be 1, 2, 4 or 8");
     }

@@ -73,9 +73,9 @@ FMCS_API size_t fmcs_workspace_bytes(const fmcs_ctx *ctx);
 FMCS_API int fmcs_profile(fmcs_ctx *ctx, int enable);
 FMCS_API int fmcs_profile_report(fmcs_ctx *ctx, char *buf, size_t len);
 /* Self-test of the bounded device waits (no reference counterpart; the
- * reference has no device code).  Every device-side wait of the library (the
- * decoupled look-backs) polls a bounded number of times, then records
- * FMCS_E_TIMEOUT in the context's status word and lets its kernel finish.
+ * reference has no device code).  A device-side wait of the library polls a
+ * bounded number of times, then records FMCS_E_TIMEOUT in the context's status
+ * word and lets its kernel finish.
  * This call runs that same wait on a word that nothing writes, with a limit of
  * `polls` polls (1..2^20), and returns what the host then reads:
  * FMCS_E_TIMEOUT, with the status word cleared and the context usable. */

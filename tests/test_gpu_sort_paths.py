@@ -84,3 +84,55 @@ def test_onchip_whole_round(ctx, n, kind):
     ng = ctx.sort_round(bank, 64, order, out_group=group)
     o, g, _, ng_ref = O.sort_round(bank)
     assert ng == ng_ref and np.array_equal(order, o) and np.array_equal(group, g)
+
+
+# Row counts around 32 tiles of 4096 (and 2048) rows, where a segment's chunk
+# rows begin to be planned in groups of 32, and a ragged larger one.
+LEVEL_SIZES = [65535, 65537, 131071, 131072, 131073, 135168, 135169, 700001]
+
+
+def _level_keys(kind, n, rng):
+    if kind == "uniform":
+        return rng.integers(0, 1 << 40, size=n, dtype=np.uint64)
+    if kind == "skip":       # the first level's digit is the same in every row: one long segment at the second
+        return rng.integers(0, 1 << 31, size=n, dtype=np.uint64)
+    if kind == "one_hot":    # nearly every row in one bucket at every level, few equal keys
+        k = rng.integers(0, 1 << 14, size=n, dtype=np.uint64)
+        far = rng.random(n) < 0.01
+        k[far] = rng.integers(0, 1 << 40, size=int(far.sum()), dtype=np.uint64)
+        return k
+    return rng.integers(0, 2, size=n, dtype=np.uint64) << np.uint64(39)   # "two": no key bits left after one level
+
+
+@pytest.mark.parametrize("n", LEVEL_SIZES)
+@pytest.mark.parametrize("kind", ["uniform", "skip", "one_hot", "two"])
+@pytest.mark.parametrize("items", [8, 16])
+def test_radix_levels(ctx, n, kind, items):
+    """HBM levels whose first histogram the stitch counts (a plan), counts
+    itself (a round), and the full-array passes."""
+    keys = _level_keys(kind, n, np.random.default_rng(n))
+    o, g, _, ng_ref = O.sort_round(keys)
+    before = ctx.get_tuning("msd_items")
+    ctx.set_tuning("msd_items", items)
+    try:
+        for how in ("plan", "round", "plain"):
+            order, group = np.zeros(n, np.uint32), np.zeros(n, np.uint32)
+            if how == "plan":
+                ng = ctx.run_plan([keys], [40], [40], order, group)
+            elif how == "round":
+                ng = ctx.sort_round(keys, 40, order, out_group=group)
+            else:
+                ng = ctx.sort_round_plain(keys, 40, order, out_group=group)
+            assert ng == ng_ref, how
+            assert np.array_equal(order, o), how
+            assert np.array_equal(group, g), how
+    finally:
+        ctx.set_tuning("msd_items", before)
+
+
+def test_radix_levels_many_segments(ctx):
+    """Large segments on both sides of 32 chunks beside each other."""
+    rng = np.random.default_rng(9)
+    sizes = [8193, 131072, 131073, 9000, 300000, 8193, 12289, 262145]
+    bank = rng.integers(0, 1 << 34, size=int(np.sum(sizes)), dtype=np.uint64)
+    _segmented(ctx, sizes, bank, 40, 3, want_keys=True)
