@@ -230,4 +230,25 @@ __device__ __forceinline__ unsigned long long lb_wait(const unsigned long long *
     return lb_word(epoch, kFlagInclusive, 0);
 }
 
+// The segment of t (prefix[s] <= t < prefix[s + 1], the last such s), found by
+// a whole warp (t the same in every lane): each round the 32 lanes probe 32
+// evenly spaced prefixes, so the range shrinks 32-fold per dependent load (two
+// rounds for 1,024 segments) instead of 2-fold as in a binary search.
+__device__ __forceinline__ uint32_t find_segment_warp(const uint32_t *prefix, uint32_t nseg, uint32_t t)
+{
+    uint32_t lo = 0, hi = nseg;  // prefix[lo] <= t < prefix[hi]
+    const uint32_t lane = lane_id();
+    while (hi - lo > 1) {
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint32_t m = lo + lane * step;
+        // the prefixes do not decrease: the lanes whose probe is <= t are a
+        // prefix of the warp, and lane 0 (probing lo) is one of them
+        const bool le = m < hi && prefix[m] <= t;
+        const uint32_t c = __popc(__ballot_sync(0xFFFFFFFFu, le));
+        lo += (c - 1) * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
 }  // namespace fmcs

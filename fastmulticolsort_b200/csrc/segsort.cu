@@ -434,27 +434,6 @@ __global__ void __launch_bounds__(1024) level_prefix_kernel(LevelRefs r)
     }
 }
 
-// The segment of tile t (tile_prefix[s] <= t < tile_prefix[s + 1]), found by
-// a whole warp (t the same in every lane): each round the 32 lanes probe 32
-// evenly spaced prefixes, so the range shrinks 32-fold per dependent load (two
-// rounds for 1,024 segments) instead of 2-fold as in a binary search.
-__device__ __forceinline__ uint32_t find_segment_warp(const uint32_t *tile_prefix, uint32_t nseg, uint32_t t)
-{
-    uint32_t lo = 0, hi = nseg;  // tile_prefix[lo] <= t < tile_prefix[hi]
-    const uint32_t lane = lane_id();
-    while (hi - lo > 1) {
-        const uint32_t step = (hi - lo + 31) / 32;
-        const uint32_t m = lo + lane * step;
-        // the prefixes do not decrease: the lanes whose probe is <= t are a
-        // prefix of the warp, and lane 0 (probing lo) is one of them
-        const bool le = m < hi && tile_prefix[m] <= t;
-        const uint32_t c = __popc(__ballot_sync(0xFFFFFFFFu, le));
-        lo += (c - 1) * step;
-        hi = min(hi, lo + step);
-    }
-    return lo;
-}
-
 // Top-digit histogram of every chunk, added to its super row as well.  A CTA
 // takes a contiguous run of chunks and reads whole ones, so a chunk's row is
 // stored, not added to.  Each thread issues all of a tile's loads before

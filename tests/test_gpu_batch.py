@@ -43,3 +43,29 @@ def test_batch_rejects_bad_instances(ctx):
     rc = L.fmcs_run_batch(ctx.handle, ptrs, capi._u32arr([2, 4]), capi._u32arr(bw), 2, capi._u32arr([32]), 1,
                           inst, 2, 100, order.ctypes.data, None, None)
     assert rc == capi.FMCS_E_INVAL
+
+
+@pytest.mark.parametrize("shift", [0, 1, 3])
+def test_batch_device_outputs_any_alignment(ctx, shift):
+    """Device outputs that start on and off a 16-byte boundary, instance borders
+    inside and at the ends of the 8,192-row steps, empty instances between."""
+    import torch
+    sizes = [8192, 0, 1, 8191, 3, 0, 0, 16381, 4096, 2, 40000, 0]
+    total = int(sum(sizes))
+    cols, bw = W.cols_uniform(total, [8, 24], seed_index=8, distinct=[3, 90])
+    dev = [torch.from_numpy(c.view({2: np.int16, 4: np.int32}[c.itemsize])).cuda() for c in cols]
+    order = torch.full((total + 8,), -7, dtype=torch.int32, device="cuda")
+    group = torch.full((total + 8,), -7, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    counts = ctx.run_batch(dev, bw, [8, 24], sizes, order[shift:shift + total], group[shift:shift + total])
+    h_order, h_group = order.cpu().numpy(), group.cpu().numpy()
+    for a in (h_order, h_group):
+        assert (a[:shift] == -7).all() and (a[shift + total:] == -7).all()
+    off = 0
+    for k, n in enumerate(sizes):
+        if n:
+            o, g, ng = O.run_plan_sort([c[off:off + n].copy() for c in cols], bw, [8, 24])
+            assert np.array_equal(h_order[shift + off:shift + off + n].view(np.uint32), o), k
+            assert np.array_equal(h_group[shift + off:shift + off + n].view(np.uint32), g), k
+            assert counts[k] == ng
+        off += n
