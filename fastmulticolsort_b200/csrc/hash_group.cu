@@ -140,20 +140,29 @@ constexpr uint32_t kDoneOnChip = 0xFFFFFFFEu;
 // Parent runs of up to kRunOnChip rows are numbered on chip (the reference's
 // block-local tables, Hashing::calculate_hash_in_block, src/hashing.h:178-287),
 // longer runs in the global table.  A classification pass (one thread per run)
-// settles one-row runs at once and queues the others by size: runs of up to
+// numbers runs of up to kRunThread rows at once, comparing every row with the
+// earlier ones in registers, and queues the others by size: runs of up to
 // 32 rows are numbered by one warp each (match.any on the key: a lane's first
 // appearance is the lowest lane holding its key), runs of 33 to kRunOnChip rows
 // by one CTA each: the run's keys are staged in shared memory, every row claims
 // or finds its key's slot of an open-addressing table of positions (at least
 // twice as many slots as rows) and lowers the slot to its own position with a
 // shared atomicMin, so a slot ends at its key's first appearance in the run.
+// kRunThread: a warp per run spends a chain of dependent loads on two or three
+// rows: the second round of 10M rows in 5M runs, 565 us in both kernels with a
+// warp for every run of 2 to 32 rows, 122 with a thread up to 8.
+constexpr uint32_t kRunThread = 8;
 constexpr uint32_t kRunOnChip = 2048;
 constexpr uint32_t kRunOnChipSlots = 2 * kRunOnChip;
 constexpr uint32_t kRunWarp = 32;
 
-__global__ void hash_runs_classify_kernel(const uint32_t *__restrict__ seg_start, const uint32_t *d_nseg,
-                                          uint32_t *slot_of, uint32_t *fpos, uint8_t *first, uint32_t *warp_runs,
-                                          uint32_t *cta_runs, uint32_t *counts)
+template <typename K>
+__global__ void __launch_bounds__(256) hash_runs_classify_kernel(const K *__restrict__ bank,
+                                                                 const uint32_t *__restrict__ order,
+                                                                 const uint32_t *__restrict__ seg_start,
+                                                                 const uint32_t *d_nseg, uint32_t *slot_of,
+                                                                 uint32_t *fpos, uint8_t *first, uint32_t *warp_runs,
+                                                                 uint32_t *cta_runs, uint32_t *counts)
 {
     kernel_prologue();
     const uint32_t nseg = *d_nseg;
@@ -172,8 +181,26 @@ __global__ void hash_runs_classify_kernel(const uint32_t *__restrict__ seg_start
             fpos[start] = start;
             first[start] = 1;
             slot_of[start] = kDoneOnChip;
+        } else if (len >= 2 && len <= kRunThread) {
+            uint32_t o[kRunThread];
+            K k[kRunThread];
+#pragma unroll
+            for (uint32_t j = 0; j < kRunThread; ++j) o[j] = j < len ? (order ? order[start + j] : start + j) : 0u;
+#pragma unroll
+            for (uint32_t j = 0; j < kRunThread; ++j) k[j] = j < len ? bank[o[j]] : K(0);
+#pragma unroll
+            for (uint32_t j = 0; j < kRunThread; ++j) {
+                if (j < len) {
+                    uint32_t f = j;   // the first row with row j's key
+#pragma unroll
+                    for (int e = (int)j - 1; e >= 0; --e) f = k[e] == k[j] ? (uint32_t)e : f;
+                    fpos[start + j] = start + f;
+                    first[start + j] = f == j ? 1 : 0;
+                    slot_of[start + j] = kDoneOnChip;
+                }
+            }
         }
-        const int which = (len >= 2 && len <= kRunWarp) ? 0 : (len > kRunWarp && len <= kRunOnChip) ? 1 : 2;
+        const int which = (len > kRunThread && len <= kRunWarp) ? 0 : (len > kRunWarp && len <= kRunOnChip) ? 1 : 2;
         const uint32_t lane = threadIdx.x & 31;
         const uint32_t peers = __match_any_sync(0xFFFFFFFFu, which);
         const uint32_t leader = __ffs(peers) - 1;
@@ -240,7 +267,7 @@ __global__ void __launch_bounds__(256) hash_runs_onchip_kernel(const K *__restri
         }
         __syncthreads();
     }
-    // runs of 2..32 rows: one warp each, lane i holding row i
+    // runs of kRunThread + 1..32 rows: one warp each, lane i holding row i
     const uint32_t nwarp = counts[0];
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t wpb = blockDim.x / 32;
@@ -316,8 +343,8 @@ int hash_insert(fmcs_ctx *ctx, const void *bank, const uint32_t *order, const ui
         cudaMemsetAsync(counts, 0, 3 * sizeof(uint32_t), ctx->stream);
         {
             LaunchScope ls_(ctx, "hash_runs_classify");
-            launch_k(hash_runs_classify_kernel, grid, 256, 0, ctx->stream, seg_start, d_nseg, slot_of, fpos, first,
-                     warp_runs, cta_runs, counts);
+            launch_k(hash_runs_classify_kernel<K>, grid, 256, 0, ctx->stream, (const K *)bank, order, seg_start, d_nseg,
+                     slot_of, fpos, first, warp_runs, cta_runs, counts);
         }
         LaunchScope ls_(ctx, "hash_runs_onchip");
         launch_k(hash_runs_onchip_kernel<K>, grid, 256, 0, ctx->stream, (const K *)bank, order, seg_start,
@@ -354,9 +381,9 @@ int hash_round(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, const uint3
     if ((rc = ws_get(ctx, kSlotHashTable, cap * sizeof(unsigned long long), &p))) return rc;
     unsigned long long *slots = (unsigned long long *)p;
     // per-row scratch: slot_of / rank, fpos, run ids, first flags; and the
-    // queues of parent runs numbered on chip (a warp each: at most n / 2 runs
-    // of 2..32 rows; a CTA each: at most n / 33)
-    const uint64_t nq_warp = n / 2 + 1, nq_cta = n / (kRunWarp + 1) + 1;
+    // queues of parent runs numbered on chip (a warp each: runs of more than
+    // kRunThread rows; a CTA each: at most n / 33)
+    const uint64_t nq_warp = n / (kRunThread + 1) + 1, nq_cta = n / (kRunWarp + 1) + 1;
     if ((rc = ws_get(ctx, kSlotHashIdx,
                      carve_total({n * sizeof(uint32_t), n * sizeof(uint32_t), n * sizeof(uint32_t), n,
                                   nq_warp * sizeof(uint32_t), nq_cta * sizeof(uint32_t)}),

@@ -136,3 +136,23 @@ def test_radix_levels_many_segments(ctx):
     sizes = [8193, 131072, 131073, 9000, 300000, 8193, 12289, 262145]
     bank = rng.integers(0, 1 << 34, size=int(np.sum(sizes)), dtype=np.uint64)
     _segmented(ctx, sizes, bank, 40, 3, want_keys=True)
+
+
+@pytest.mark.parametrize("last", [False, True])
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.uint32, np.uint64])
+def test_hash_runs_by_size(ctx, dtype, last):
+    """Parent runs on both sides of every way of numbering them (a thread up to
+    8 rows, a warp up to 32, a CTA up to 2048, the table beyond)."""
+    rng = np.random.default_rng(dtype().itemsize)
+    sizes = [int(x) for x in rng.permutation([1, 2, 3, 7, 8, 9, 31, 32, 33, 2047, 2048, 2049] * 3)]
+    n = int(np.sum(sizes))
+    in_group = np.repeat(np.arange(len(sizes), dtype=np.uint32), sizes)
+    bank = (rng.integers(0, 5, size=n) * 37).astype(dtype)
+    order_in = rng.permutation(n).astype(np.uint32)
+    order, group = order_in.copy(), np.zeros(n, np.uint32)
+    ng = ctx.hash_round(bank, order, in_group=in_group, out_group=group, last_round=last)
+    o, g, ids, ng_ref = O.hash_round(bank, order=order_in, in_group=in_group, last_round=last)
+    g = ids if last else g   # the last round leaves the ids at their positions
+    assert ng == ng_ref
+    assert np.array_equal(order, o)
+    assert np.array_equal(group, g)
