@@ -147,6 +147,21 @@ int plan_pipeline(fmcs_ctx *ctx, const Plan &plan, const void *const *dcols, con
     uint32_t *w;
     if ((rc = counters(ctx, &w))) return rc;
     uint32_t *d_ng = w + kCtrNgroups;
+    if (!hash) {
+        // few rows: the whole plan in one launch
+        std::vector<StitchSlice> sl;
+        std::vector<int> ns;
+        for (const BankPlan &bp : plan.banks) {
+            ns.push_back((int)bp.slices.size());
+            for (const SliceRec &sr : bp.slices)
+                sl.push_back(StitchSlice{dcols[sr.col], col_bytes[sr.col], bw[sr.col] - sr.end, sr.end - sr.start + 1,
+                                         descending && descending[sr.col] ? 1u : 0u});
+        }
+        if (small_plan_fits(n, ns.data(), nbanks)) {
+            *d_ng_out = d_ng;
+            return launch_small_plan(ctx, sl.data(), ns.data(), nbanks, n, dorder, dgroup_out, d_ng);
+        }
+    }
     // group ping-pong and segment starts
     uint32_t *g[2];
     if ((rc = ws_get(ctx, kSlotGroupA, n * 4, &p))) return rc;
@@ -381,9 +396,13 @@ extern "C" int fmcs_sort_round(fmcs_ctx *ctx, const void *bank, uint32_t bank_by
     uint32_t *w;
     if ((rc = counters(ctx, &w))) return rc;
     uint32_t *d_ng = w + kCtrNgroups;
-    if ((rc = sort_round_dev(ctx, dbank, bank_bytes, key_bits, (uint32_t *)dorder, (const uint32_t *)dig, nullptr,
-                             nullptr, (uint32_t *)dgroup, dkeys, nullptr, nullptr, n, d_ng)))
-        return rc;
+    if (n <= kSmallRows)
+        rc = launch_small_round(ctx, dbank, bank_bytes, key_bits, dig ? (const uint32_t *)dorder : nullptr,
+                                (const uint32_t *)dig, (uint32_t *)dorder, (uint32_t *)dgroup, dkeys, n, d_ng);
+    else
+        rc = sort_round_dev(ctx, dbank, bank_bytes, key_bits, (uint32_t *)dorder, (const uint32_t *)dig, nullptr,
+                            nullptr, (uint32_t *)dgroup, dkeys, nullptr, nullptr, n, d_ng);
+    if (rc) return rc;
     if (h_order && (rc = copy_out(ctx, order, dorder, n * 4))) return rc;
     if (h_group && (rc = copy_out(ctx, out_group, dgroup, n * 4))) return rc;
     if (h_keys && (rc = copy_out(ctx, sorted_bank, dkeys, n * bank_bytes))) return rc;

@@ -253,6 +253,18 @@ constexpr uint32_t kTopSuper = 32;
 // [0, bits): the plain, unsegmented comparator path.
 int lsd_sort_full(fmcs_ctx *ctx, void *keys, uint32_t key_bytes, uint32_t *vals, uint64_t n, uint32_t bits);
 
+// ---------------------------------------------------------------- small plans
+// A whole sort plan or round over at most kSmallRows rows in one launch
+// (small.cu).  slices: every bank's slices, bank after bank (nslices[b] of
+// bank b).
+constexpr uint64_t kSmallRows = 8192;
+bool small_plan_fits(uint64_t n, const int *nslices, uint32_t nbanks);
+int launch_small_plan(fmcs_ctx *ctx, const StitchSlice *slices, const int *nslices, uint32_t nbanks, uint64_t n,
+                      uint32_t *order_out, uint32_t *group_out, uint32_t *d_ngroups);
+int launch_small_round(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, uint32_t key_bits, const uint32_t *order_in,
+                       const uint32_t *in_group, uint32_t *order_out, uint32_t *group_out, void *keys_out, uint64_t n,
+                       uint32_t *d_ngroups);
+
 // ---------------------------------------------------------------- group ids / segments
 // out_group[i] = number of boundaries in (0, i], boundary at i when
 // keys[i] != keys[i-1] or (in_group && in_group[i] != in_group[i-1]).

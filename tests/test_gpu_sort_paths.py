@@ -156,3 +156,49 @@ def test_hash_runs_by_size(ctx, dtype, last):
     assert ng == ng_ref
     assert np.array_equal(order, o)
     assert np.array_equal(group, g)
+
+
+SMALL = [1, 2, 31, 32, 33, 255, 256, 257, 1023, 1024, 1025, 4095, 4096, 4097, 8191, 8192, 8193]
+
+
+@pytest.mark.parametrize("n", SMALL)
+@pytest.mark.parametrize("split", [[64], [1, 63], [5, 30, 29], [16, 16, 16, 16]])
+def test_small_plans(ctx, n, split):
+    """Plans around the one-launch limit (8192 rows), with repeated codes,
+    a descending column and a captured graph."""
+    import torch
+    rng = np.random.default_rng(n + len(split))
+    bw = [12, 31, 21]
+    cols = [(rng.integers(0, 3, size=n) * 1365).astype(np.uint16),
+            rng.integers(0, 1 << 31, size=n, dtype=np.uint64).astype(np.uint32) % np.uint32(1 + n // 2),
+            rng.integers(0, 1 << 21, size=n, dtype=np.uint64).astype(np.uint32)]
+    order, group = np.zeros(n, np.uint32), np.zeros(n, np.uint32)
+    for desc in (None, [0, 1, 0]):
+        ng = ctx.run_plan(cols, bw, split, order, group, descending=desc)
+        flip = [np.asarray((1 << w) - 1 - c.astype(np.int64)).astype(c.dtype) if desc and desc[k] else c
+                for k, (c, w) in enumerate(zip(cols, bw))]
+        o, g, ng_ref = O.run_plan_sort(flip, bw, split)
+        assert ng == ng_ref and np.array_equal(order, o) and np.array_equal(group, g)
+    dev = [torch.from_numpy(c.view({2: np.int16, 4: np.int32}[c.itemsize])).cuda() for c in cols]
+    d_order, d_group = (torch.zeros(n, dtype=torch.int32, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    graph = ctx.plan_graph(dev, bw, split, d_order, d_group)
+    o, g, ng_ref = O.run_plan_sort(cols, bw, split)
+    for _ in range(2):
+        assert graph.launch() == ng_ref
+        assert np.array_equal(d_order.cpu().numpy().view(np.uint32), o)
+        assert np.array_equal(d_group.cpu().numpy().view(np.uint32), g)
+    graph.close()
+
+
+@pytest.mark.parametrize("n", SMALL)
+@pytest.mark.parametrize("dtype,bits", [(np.uint16, 9), (np.uint32, 32), (np.uint64, 64)])
+def test_small_segmented_rounds(ctx, n, dtype, bits):
+    """Segmented rounds around the same limit; a previous order that is not
+    ascending inside its segments."""
+    rng = np.random.default_rng(n)
+    cuts = np.sort(rng.choice(np.arange(1, n), size=min(n - 1, n // 3), replace=False)) if n > 1 else np.array([], int)
+    sizes = np.diff(np.concatenate([[0], cuts, [n]]))
+    bank = (rng.integers(0, 1 << 9, size=n, dtype=np.uint64) % np.uint64(7)).astype(dtype)
+    _segmented(ctx, sizes, bank, bits, n, want_keys=True)
+    _segmented(ctx, [n], bank, bits, n)
