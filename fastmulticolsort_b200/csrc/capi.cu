@@ -5,7 +5,7 @@
 // src/stitch_composer.cpp:684-687), host<->device staging for host pointers,
 // the round loop of Composer::multiRoundSorting (src/composer.cpp:48-135) and
 // of StitchComposer::run_single_plan (src/stitch_composer.cpp:555-806), and the
-// final status check of the bounded device waits.
+// hand-over of status and group count to the host.
 #include "device_common.cuh"
 #include "fmcs_internal.h"
 #include "plan.h"
@@ -64,18 +64,8 @@ int copy_out(fmcs_ctx *ctx, void *host, const void *dev, size_t bytes)
 
 bool valid_bank(uint32_t b) { return b == 1 || b == 2 || b == 4 || b == 8; }
 
-int finish(fmcs_ctx *ctx, const char *what, uint32_t *ngroups, const uint32_t *d_ng)
-{
-    if (ngroups && d_ng) {
-        cudaError_t e = cudaMemcpyAsync(ctx->h_small + 1, d_ng, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                        ctx->stream);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, what);
-    }
-    int rc = check_status(ctx, what);   // synchronizes
-    if (rc) return rc;
-    if (ngroups) *ngroups = d_ng ? ctx->h_small[1] : 0;
-    return FMCS_OK;
-}
+// Where a sort plan's last scan stores its group count: the host's word itself.
+uint32_t *host_ngroups(fmcs_ctx *ctx) { return ctx->h_small + kHostNgroups; }
 
 int counters(fmcs_ctx *ctx, uint32_t **w)
 {
@@ -136,17 +126,17 @@ int sort_round_dev(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, uint32_
 // The device work of one plan (stitch + rounds), enqueued on the context's
 // stream with no host synchronization when `fixed` (every radix level is
 // launched and exits on the device when it has nothing to do): the form a
-// CUDA graph captures.  *d_ng_out receives the device word of the group count.
+// CUDA graph captures.  The group count ends in the host's word.
 int plan_pipeline(fmcs_ctx *ctx, const Plan &plan, const void *const *dcols, const uint32_t *col_bytes,
                   const uint32_t *bw, uint64_t n, bool hash, uint32_t *dorder, uint32_t *dgroup_out, bool fixed,
-                  uint32_t **d_ng_out, const uint8_t *descending = nullptr)
+                  const uint8_t *descending = nullptr)
 {
     int rc;
     void *p;
     const uint32_t nbanks = (uint32_t)plan.banks.size();
     uint32_t *w;
     if ((rc = counters(ctx, &w))) return rc;
-    uint32_t *d_ng = w + kCtrNgroups;
+    uint32_t *d_ng = hash ? w + kCtrNgroups : host_ngroups(ctx);   // (hash rounds read it on the device)
     if (!hash) {
         // few rows: the whole plan in one launch
         std::vector<StitchSlice> sl;
@@ -158,7 +148,6 @@ int plan_pipeline(fmcs_ctx *ctx, const Plan &plan, const void *const *dcols, con
                                          descending && descending[sr.col] ? 1u : 0u});
         }
         if (small_plan_fits(n, ns.data(), nbanks)) {
-            *d_ng_out = d_ng;
             return launch_small_plan(ctx, sl.data(), ns.data(), nbanks, n, dorder, dgroup_out, d_ng);
         }
     }
@@ -247,8 +236,7 @@ int plan_pipeline(fmcs_ctx *ctx, const Plan &plan, const void *const *dcols, con
         in_group = og;
     }
     ctx->prof_round = -1;
-    *d_ng_out = d_ng;
-    return FMCS_OK;
+    return hash ? publish(ctx, d_ng) : FMCS_OK;
 }
 
 }  // namespace
@@ -296,7 +284,7 @@ extern "C" int fmcs_stitch(fmcs_ctx *ctx, const fmcs_slice *slices, uint32_t nsl
     if ((rc = stage_out(ctx, bank, n * bank_bytes, kSlotStageOut0, &dbank, &host_out))) return rc;
     if ((rc = launch_stitch(ctx, sl.data(), (int)nslices, dbank, bank_bytes, n))) return rc;
     if (host_out && (rc = copy_out(ctx, bank, dbank, n * bank_bytes))) return rc;
-    return finish(ctx, "fmcs_stitch", nullptr, nullptr);
+    return finish(ctx, "fmcs_stitch", nullptr);
 }
 
 extern "C" int fmcs_shift_left(fmcs_ctx *ctx, void *bank, uint32_t bank_bytes, uint64_t n, uint32_t nbits)
@@ -316,7 +304,7 @@ extern "C" int fmcs_shift_left(fmcs_ctx *ctx, void *bank, uint32_t bank_bytes, u
     }
     if ((rc = launch_bank_update(ctx, dbank, bank_bytes, n, nbits, nullptr, 0, 0, 0))) return rc;
     if (host && (rc = copy_out(ctx, bank, dbank, n * bank_bytes))) return rc;
-    return finish(ctx, "fmcs_shift_left", nullptr, nullptr);
+    return finish(ctx, "fmcs_shift_left", nullptr);
 }
 
 extern "C" int fmcs_assemble(fmcs_ctx *ctx, void *bank, uint32_t bank_bytes, uint64_t n, const fmcs_slice *s)
@@ -342,7 +330,7 @@ extern "C" int fmcs_assemble(fmcs_ctx *ctx, void *bank, uint32_t bank_bytes, uin
                                  s->end - s->start + 1)))
         return rc;
     if (host && (rc = copy_out(ctx, bank, dbank, n * bank_bytes))) return rc;
-    return finish(ctx, "fmcs_assemble", nullptr, nullptr);
+    return finish(ctx, "fmcs_assemble", nullptr);
 }
 
 extern "C" int fmcs_gather(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, const uint32_t *order, void *out,
@@ -363,7 +351,7 @@ extern "C" int fmcs_gather(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes,
     if ((rc = stage_out(ctx, out, n * bank_bytes, kSlotStageOut0, &dout, &host_out))) return rc;
     if ((rc = launch_gather(ctx, dbank, bank_bytes, (const uint32_t *)dorder, dout, n))) return rc;
     if (host_out && (rc = copy_out(ctx, out, dout, n * bank_bytes))) return rc;
-    return finish(ctx, "fmcs_gather", nullptr, nullptr);
+    return finish(ctx, "fmcs_gather", nullptr);
 }
 
 extern "C" int fmcs_sort_round(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, uint32_t key_bits,
@@ -393,9 +381,7 @@ extern "C" int fmcs_sort_round(fmcs_ctx *ctx, const void *bank, uint32_t bank_by
     }
     if ((rc = stage_out(ctx, out_group, n * 4, kSlotStageOut1, &dgroup, &h_group))) return rc;
     if ((rc = stage_out(ctx, sorted_bank, n * bank_bytes, kSlotStageOut2, &dkeys, &h_keys))) return rc;
-    uint32_t *w;
-    if ((rc = counters(ctx, &w))) return rc;
-    uint32_t *d_ng = w + kCtrNgroups;
+    uint32_t *d_ng = host_ngroups(ctx);
     if (n <= kSmallRows)
         rc = launch_small_round(ctx, dbank, bank_bytes, key_bits, dig ? (const uint32_t *)dorder : nullptr,
                                 (const uint32_t *)dig, (uint32_t *)dorder, (uint32_t *)dgroup, dkeys, n, d_ng);
@@ -406,7 +392,7 @@ extern "C" int fmcs_sort_round(fmcs_ctx *ctx, const void *bank, uint32_t bank_by
     if (h_order && (rc = copy_out(ctx, order, dorder, n * 4))) return rc;
     if (h_group && (rc = copy_out(ctx, out_group, dgroup, n * 4))) return rc;
     if (h_keys && (rc = copy_out(ctx, sorted_bank, dkeys, n * bank_bytes))) return rc;
-    return finish(ctx, "fmcs_sort_round", ngroups, out_group ? d_ng : nullptr);
+    return finish(ctx, "fmcs_sort_round", out_group ? ngroups : nullptr);
 }
 
 extern "C" int fmcs_sort_round_plain(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, uint32_t key_bits,
@@ -440,9 +426,7 @@ extern "C" int fmcs_sort_round_plain(fmcs_ctx *ctx, const void *bank, uint32_t b
     if ((rc = ws_get(ctx, kSlotMisc, 3 * carve_round(n * sizeof(uint32_t)), &p))) return rc;
     Carver cv(p);
     uint32_t *pos = cv.take<uint32_t>(n), *grp = cv.take<uint32_t>(n), *tmp = cv.take<uint32_t>(n);
-    uint32_t *w;
-    if ((rc = counters(ctx, &w))) return rc;
-    uint32_t *d_ng = w + kCtrNgroups;
+    uint32_t *d_ng = host_ngroups(ctx);
     cudaStream_t st = ctx->stream;
     // keys of this round in the previous order, positions as payload
     if (in_group) {
@@ -455,11 +439,11 @@ extern "C" int fmcs_sort_round_plain(fmcs_ctx *ctx, const void *bank, uint32_t b
     if ((rc = lsd_sort_full(ctx, kg, bank_bytes, pos, n, key_bits))) return rc;
     if (in_group) {
         if ((rc = launch_gather(ctx, dig, 4, pos, grp, n))) return rc;
-        cudaMemcpyAsync(ctx->h_small + 2, (const uint32_t *)dig + (n - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(ctx->h_small + kHostSpare, (const uint32_t *)dig + (n - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
         cudaError_t e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "fmcs_sort_round_plain sync");
         uint32_t gbits = 1;
-        while (gbits < 32 && (1ull << gbits) <= (uint64_t)ctx->h_small[2]) gbits++;
+        while (gbits < 32 && (1ull << gbits) <= (uint64_t)ctx->h_small[kHostSpare]) gbits++;
         if ((rc = lsd_sort_full(ctx, grp, 4, pos, n, gbits))) return rc;
         // order_out[i] = order_in[pos[i]]
         cudaMemcpyAsync(tmp, dorder, n * 4, cudaMemcpyDeviceToDevice, st);
@@ -474,7 +458,7 @@ extern "C" int fmcs_sort_round_plain(fmcs_ctx *ctx, const void *bank, uint32_t b
     if (h_order && (rc = copy_out(ctx, order, dorder, n * 4))) return rc;
     if (h_group && (rc = copy_out(ctx, out_group, dgroup, n * 4))) return rc;
     if (h_keys && (rc = copy_out(ctx, sorted_bank, dkeys, n * bank_bytes))) return rc;
-    return finish(ctx, "fmcs_sort_round_plain", ngroups, out_group ? d_ng : nullptr);
+    return finish(ctx, "fmcs_sort_round_plain", out_group ? ngroups : nullptr);
 }
 
 extern "C" int fmcs_hash_round(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, uint32_t *order,
@@ -516,7 +500,8 @@ extern "C" int fmcs_hash_round(fmcs_ctx *ctx, const void *bank, uint32_t bank_by
         return rc;
     if (h_order && (rc = copy_out(ctx, order, dorder, n * 4))) return rc;
     if (h_group && (rc = copy_out(ctx, out_group, dgroup, n * 4))) return rc;
-    return finish(ctx, "fmcs_hash_round", ngroups, d_ng);
+    if ((rc = publish(ctx, d_ng))) return rc;
+    return finish(ctx, "fmcs_hash_round", ngroups);
 }
 
 extern "C" int fmcs_hash_round_unordered(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes,
@@ -545,7 +530,8 @@ extern "C" int fmcs_hash_round_unordered(fmcs_ctx *ctx, const void *bank, uint32
                          d_ng, true)))
         return rc;
     if (h_group && (rc = copy_out(ctx, out_group, dgroup, n * 4))) return rc;
-    return finish(ctx, "fmcs_hash_round_unordered", ngroups, d_ng);
+    if ((rc = publish(ctx, d_ng))) return rc;
+    return finish(ctx, "fmcs_hash_round_unordered", ngroups);
 }
 
 namespace {
@@ -601,14 +587,13 @@ int run_plan_impl(fmcs_ctx *ctx, const void *const *cols, const uint32_t *col_by
     bool h_order, h_group;
     if ((rc = stage_out(ctx, order_out, n * 4, kSlotStageOut0, &dorder, &h_order))) return rc;
     if ((rc = stage_out(ctx, group_out, n * 4, kSlotStageOut1, &dgroup_out, &h_group))) return rc;
-    uint32_t *d_ng = nullptr;
     if ((rc = plan_pipeline(ctx, plan, dcols.data(), col_bytes, bw, n, hash != 0, (uint32_t *)dorder,
-                            (uint32_t *)dgroup_out, false, &d_ng, descending)))
+                            (uint32_t *)dgroup_out, false, descending)))
         return rc;
     ctx->prof_round = -1;
     if (h_order && (rc = copy_out(ctx, order_out, dorder, n * 4))) return rc;
     if (h_group && (rc = copy_out(ctx, group_out, dgroup_out, n * 4))) return rc;
-    return finish(ctx, "fmcs_run_plan", ngroups, d_ng);
+    return finish(ctx, "fmcs_run_plan", ngroups);
 }
 }  // namespace
 
@@ -890,7 +875,7 @@ extern "C" int fmcs_run_batch(fmcs_ctx *ctx, const void *const *cols, const uint
     }
     if (h_order && (rc = copy_out(ctx, order_out, dorder, n * 4))) return rc;
     if (h_group && (rc = copy_out(ctx, group_out, dgroup_out, n * 4))) return rc;
-    return finish(ctx, "fmcs_run_batch", nullptr, nullptr);
+    return finish(ctx, "fmcs_run_batch", nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -900,7 +885,6 @@ struct fmcs_graph {
     fmcs_ctx *ctx = nullptr;   // private context: its workspace stays as captured
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    uint32_t *d_ng = nullptr;
     unsigned long long kernels = 0;   // kernel nodes captured (a loop body once)
 };
 
@@ -948,14 +932,14 @@ static int graph_create(fmcs_ctx *parent, const void *const *cols, const uint32_
     ctx->local_max = parent->local_max;
     ctx->msd_items = parent->msd_items;
     // 1) one eager run of the fixed launch sequence sizes every workspace slot
-    rc = plan_pipeline(ctx, plan, cols, col_bytes, bw, n, hash, order_out, group_out, true, &g->d_ng);
+    rc = plan_pipeline(ctx, plan, cols, col_bytes, bw, n, hash, order_out, group_out, true);
     if (!rc) rc = check_status(ctx, "fmcs_graph_create warm-up");
     // 2) capture the same launches
     if (!rc) {
         cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
             const unsigned long long l0 = ctx->launches;   // every launch site counts itself
-            rc = plan_pipeline(ctx, plan, cols, col_bytes, bw, n, hash, order_out, group_out, true, &g->d_ng);
+            rc = plan_pipeline(ctx, plan, cols, col_bytes, bw, n, hash, order_out, group_out, true);
             g->kernels = ctx->launches - l0;
             cudaGraph_t graph = nullptr;
             e = cudaStreamEndCapture(ctx->stream, &graph);
@@ -997,7 +981,7 @@ extern "C" int fmcs_graph_launch(fmcs_graph *g, uint32_t *ngroups)
     cudaSetDevice(g->ctx->device);
     cudaError_t e = cudaGraphLaunch(g->exec, g->ctx->stream);
     if (e != cudaSuccess) return cuda_fail(g->ctx, e, "fmcs_graph_launch");
-    return finish(g->ctx, "fmcs_graph_launch", ngroups, g->d_ng);
+    return finish(g->ctx, "fmcs_graph_launch", ngroups);
 }
 
 extern "C" void *fmcs_graph_stream(fmcs_graph *g) { return g && g->ctx ? (void *)g->ctx->stream : nullptr; }

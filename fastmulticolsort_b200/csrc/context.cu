@@ -7,6 +7,7 @@
 
 #include <dlfcn.h>
 
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <fstream>
@@ -137,16 +138,64 @@ int capture_while(fmcs_ctx *ctx, cudaStream_t st,
     return FMCS_OK;
 }
 
-int check_status(fmcs_ctx *ctx, const char *what)
+namespace {
+// The status word and (d_ng != NULL) a group count to the host's words; a status
+// is handed over once.
+__global__ void publish_kernel(int *d_status, const uint32_t *d_ng, uint32_t *host)
 {
-    cudaError_t e = cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost,
-                                    ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    kernel_prologue();
+    if (threadIdx.x == 0) {
+        const int s = *d_status;
+        host[kHostStatus] = (uint32_t)s;
+        if (s != 0) *d_status = 0;
+        if (d_ng) host[kHostNgroups] = *d_ng;
+    }
+}
+
+// The sort engine's counters to the host's words, then their sequence number.
+__global__ void publish_counters_kernel(const uint32_t *ctr, uint32_t *host, uint32_t seq)
+{
+    kernel_prologue();
+    publish_counters(ctr, host, seq);
+}
+}  // namespace
+
+int publish(fmcs_ctx *ctx, const uint32_t *d_ng)
+{
+    LaunchScope ls_(ctx, "publish");
+    const cudaError_t e = launch_k(publish_kernel, 1, 32, 0, ctx->stream, ctx->d_status, d_ng, ctx->h_small);
+    return e == cudaSuccess ? FMCS_OK : cuda_fail(ctx, e, "publish launch");
+}
+
+int launch_publish_counters(fmcs_ctx *ctx, const uint32_t *ctr, uint32_t seq)
+{
+    LaunchScope ls_(ctx, "publish");
+    const cudaError_t e = launch_k(publish_counters_kernel, 1, 32, 0, ctx->stream, ctr, ctx->h_small, seq);
+    return e == cudaSuccess ? FMCS_OK : cuda_fail(ctx, e, "publish launch");
+}
+
+int wait_counters(fmcs_ctx *ctx, uint32_t seq, const char *what)
+{
+    volatile const uint32_t *at = ctx->h_small + kHostSeq;
+    for (uint32_t it = 1; *at != seq; ++it) {
+        if ((it & 1023u) != 0) continue;
+        // now and then: has the stream failed, or ended without the counters?
+        const cudaError_t e = cudaStreamQuery(ctx->stream);
+        if (e == cudaErrorNotReady) continue;
+        if (e != cudaSuccess) return cuda_fail(ctx, e, what);
+        if (*at != seq) return set_error(ctx, FMCS_E_CUDA, std::string(what) + ": no counters");
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return FMCS_OK;
+}
+
+int finish(fmcs_ctx *ctx, const char *what, uint32_t *ngroups)
+{
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, what);
-    int s = *ctx->h_status;
+    const int s = (int)ctx->h_small[kHostStatus];
     if (s != 0) {
-        *ctx->h_status = 0;
-        cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);
+        ctx->h_small[kHostStatus] = 0;
         char buf[200];
         if (s == FMCS_E_TIMEOUT)
             snprintf(buf, sizeof(buf), "%s: a device-side wait timed out", what);
@@ -154,7 +203,14 @@ int check_status(fmcs_ctx *ctx, const char *what)
             snprintf(buf, sizeof(buf), "%s: device reported status %d", what, s);
         return set_error(ctx, s == FMCS_E_TIMEOUT ? FMCS_E_TIMEOUT : FMCS_E_INVAL, buf);
     }
+    if (ngroups) *ngroups = ctx->h_small[kHostNgroups];
     return FMCS_OK;
+}
+
+int check_status(fmcs_ctx *ctx, const char *what)
+{
+    const int rc = publish(ctx, nullptr);
+    return rc ? rc : finish(ctx, what, nullptr);
 }
 
 static cudaEvent_t take_event(fmcs_ctx *ctx)
@@ -273,9 +329,7 @@ extern "C" int fmcs_create(fmcs_ctx **out, int device, size_t hbm_budget_bytes)
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_status, 256);
     if (e == cudaSuccess) e = cudaMemset(ctx->d_status, 0, 256);
-    if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_status, sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_small, 64 * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_level, cudaEventDisableTiming);
     // the second stream and its events exist from the start, so that a call
     // made while the caller captures the context's stream creates nothing
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->par, cudaStreamNonBlocking);
@@ -286,7 +340,7 @@ extern "C" int fmcs_create(fmcs_ctx **out, int device, size_t hbm_budget_bytes)
         fmcs_destroy(ctx);
         return FMCS_E_CUDA;
     }
-    *ctx->h_status = 0;
+    memset(ctx->h_small, 0, 64 * sizeof(uint32_t));
     load_tuning(ctx);
     if (const char *m = getenv("FMCS_RANK_MODE"))
         ctx->rank_mode = (m[0] == 'b' || m[0] == '1') ? 1 : (m[0] == 'o' || m[0] == '2') ? 2 : 0;
@@ -307,9 +361,7 @@ extern "C" void fmcs_destroy(fmcs_ctx *ctx)
     }
     for (auto e : ctx->ev_pool) cudaEventDestroy(e);
     if (ctx->d_status) cudaFree(ctx->d_status);
-    if (ctx->h_status) cudaFreeHost(ctx->h_status);
     if (ctx->h_small) cudaFreeHost(ctx->h_small);
-    if (ctx->ev_level) cudaEventDestroy(ctx->ev_level);
     if (ctx->side) cudaStreamDestroy(ctx->side);
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);

@@ -251,4 +251,26 @@ __device__ __forceinline__ uint32_t find_segment_warp(const uint32_t *prefix, ui
     return lo;
 }
 
+// The words of the host's pinned page that kernels write (fmcs_ctx::h_small): a
+// status, a group count, and the sort engine's counters with the number of the
+// read-back they belong to.  A copy engine's turn on the stream costs 6 to 10 us,
+// a store 1.
+constexpr int kHostStatus = 0;
+constexpr int kHostNgroups = 1;
+constexpr int kHostSeq = 2;
+constexpr int kHostSpare = 3;   // (a copy's target)
+constexpr int kHostCounters = 16;
+constexpr int kHostCounterWords = 32;
+
+// The calling warp stores the counters, then (after they are visible to the
+// host) the sequence number.
+__device__ __forceinline__ void publish_counters(const uint32_t *ctr, uint32_t *host, uint32_t seq)
+{
+    const uint32_t lane = lane_id();
+    *(volatile uint32_t *)&host[kHostCounters + lane] = *(volatile const uint32_t *)&ctr[lane];
+    __threadfence_system();
+    __syncwarp();
+    if (lane == 0) *(volatile uint32_t *)&host[kHostSeq] = seq;
+}
+
 }  // namespace fmcs

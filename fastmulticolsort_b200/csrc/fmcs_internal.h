@@ -82,14 +82,13 @@ struct fmcs_ctx {
     fmcs::Workspace ws;
     int *d_status = nullptr;       // device status word
     std::string err;
-    int *h_status = nullptr;       // pinned mirror of the status word
-    uint32_t *h_small = nullptr;   // pinned small read-back area (64 words)
+    uint32_t *h_small = nullptr;   // pinned words that kernels write for the host (kHost* in device_common.cuh)
+    uint32_t read_backs = 0;       // sequence number of the last counter read-back
     // kernel profiler: CUDA events around every launch while enabled
     bool prof_on = false;
     std::vector<fmcs_prof_rec> prof;
     std::vector<cudaEvent_t> ev_pool;
     unsigned long long launches = 0;   // kernels launched by this context
-    cudaEvent_t ev_level = nullptr;    // host-side read-back point of the sort levels
     // tuned knobs (the autotuner's tuning/b200.json, FMCS_TUNING, or fmcs_set_tuning)
     int rank_mode = 0;                 // 0: match.any multi-split, 1: ballot, 2: shared-memory OR
     uint32_t local_max = 8192;         // segments above this many rows take the MSD levels
@@ -131,8 +130,19 @@ int set_error(fmcs_ctx *ctx, int code, const std::string &msg);
 int cuda_fail(fmcs_ctx *ctx, cudaError_t e, const char *what);
 // Returns a device pointer of at least `bytes` in `slot` (grown as needed).
 int ws_get(fmcs_ctx *ctx, int slot, size_t bytes, void **out);
+// Enqueues the hand-over of the device status word (and a group count) to the
+// host's words; calls whose kernels can set a status end with it.
+int publish(fmcs_ctx *ctx, const uint32_t *d_ng);
+// Waits for the stream; a status handed over becomes the return code.  ngroups
+// (optional) receives the host's group count word.
+int finish(fmcs_ctx *ctx, const char *what, uint32_t *ngroups);
 // Checks and clears the device status word (synchronizes the stream).
 int check_status(fmcs_ctx *ctx, const char *what);
+// Read-back number `seq` of the sort engine's counters (32 device words): a
+// launch that stores them for the host, and the host's wait for it (or for
+// another kernel that calls publish_counters).
+int launch_publish_counters(fmcs_ctx *ctx, const uint32_t *ctr, uint32_t seq);
+int wait_counters(fmcs_ctx *ctx, uint32_t seq, const char *what);
 
 // Brackets one kernel launch: counts it and, while profiling is on, records
 // a pair of CUDA events on the context's stream around it.

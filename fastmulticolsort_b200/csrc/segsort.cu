@@ -81,7 +81,7 @@ constexpr int kCtrLocalC3 = 16;
 constexpr int kCtrLocalC1b = 17;
 constexpr int kCtrWork = 18;       // chunks the current level's scatter moves
 constexpr int kCtrLong = 19;       // super rows of the level's long segments (level_prefix_kernel)
-constexpr int kCtrWords = 32;
+constexpr int kCtrWords = kHostCounterWords;
 
 // An HBM level cuts each large segment into chunks of a few tiles (chunk_rows
 // rows, msd_chunk_rows).  A chunk has its own histogram row, counted by the CTA
@@ -680,7 +680,8 @@ struct MsdSmem {
 template <typename K, int RANK, int IT>
 __global__ void __launch_bounds__(kNtM, msd_ctas_per_sm(IT)) msd_scatter_kernel(Bufs<K> b, LevelRefs r,
                                                                                 cudaGraphConditionalHandle more,
-                                                                                uint32_t levels)
+                                                                                uint32_t levels, uint32_t *host,
+                                                                                uint32_t seq)
 {
     kernel_prologue();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -688,6 +689,9 @@ __global__ void __launch_bounds__(kNtM, msd_ctas_per_sm(IT)) msd_scatter_kernel(
     constexpr uint32_t kTileM = kNtM * IT;
     const uint32_t lvl = running_level(r);
     const uint32_t cur = lvl & 1u;
+    // An eager call reads the counters back (the next level's count, the rows
+    // moved, the tiers' list sizes, final since msd_plan) while this kernel runs.
+    if (host && blockIdx.x == 0 && threadIdx.x < 32) publish_counters(r.ctr, host, seq);
     // Inside a graph, the level loop goes on while the next level has large
     // segments (msd_plan has counted them before this launch).
     const uint32_t nnext = r.ctr[kCtrLarge0 + (cur ^ 1u)];
@@ -1137,13 +1141,13 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
         }
         FMCS_LAUNCH_CHECK("classify");
     }
-    // The host's copy of the counters (ctx->h_small + 16) when an eager call
+    // The host's copy of the counters when an eager call
     // has read them back after the last routing of segments to the tiers.
     bool tiers_known = false;
-    const uint32_t *hctr = ctx->h_small + 16;
+    uint32_t *hctr = ctx->h_small + kHostCounters;
     if (!a.fixed_launches && !a.seg_start && !a.d_key_bits && !a.d_in_order && n <= (uint64_t)local_max) {
         // round 0 that fits one tier: the host routes it as classify does
-        uint32_t *w = ctx->h_small + 16;
+        uint32_t *w = hctr;
         for (int i = 0; i < kCtrWords; ++i) w[i] = 0;
         const uint32_t len = (uint32_t)n;
         if (len > 1) {
@@ -1160,6 +1164,13 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
         }
         tiers_known = true;
     }
+    if (!a.fixed_launches && a.seg_start) {
+        // how many segments each way of sorting them got
+        const uint32_t seq = ++ctx->read_backs;
+        if ((rc = launch_publish_counters(ctx, ctr, seq))) return rc;
+        if ((rc = wait_counters(ctx, seq, "sort: segment counts"))) return rc;
+        tiers_known = true;
+    }
     // MSD levels
     const int levels = (int)((a.key_bits + kRadixBits - 1) / kRadixBits);
     const size_t msd_smem = sizeof(MsdSmem<K, IT>);
@@ -1167,16 +1178,7 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
     if (n > (uint64_t)local_max) {
         // Host-known count of the level's large segments (exact unless the
         // caller asked for a fixed launch sequence, e.g. for graph capture).
-        uint32_t nlarge = 1;
-        if (a.fixed_launches) {
-            nlarge = 1;
-        } else if (a.seg_start) {
-            cudaMemcpyAsync(ctx->h_small + 16, ctr, kCtrWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-            cudaError_t e = cudaStreamSynchronize(st);
-            if (e != cudaSuccess) return cuda_fail(ctx, e, "sort: level count");
-            nlarge = ctx->h_small[16 + kCtrLarge0];
-            tiers_known = true;
-        }
+        uint32_t nlarge = a.fixed_launches || !a.seg_start ? 1u : hctr[kCtrLarge0];
         const unsigned scatter_grid = sms * msd_ctas_per_sm(IT);
         int host_lvl = 0;   // the level being launched, for the eager read-back
         // one level: the same four launches for every level (the level index
@@ -1193,23 +1195,18 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
             { LaunchScope ls_(ctx, "msd_plan");
                 launch_k(msd_plan_kernel, sms * 8, kPlanThreads, 0, s, lr, lists, true);
             }
-            if (read_back) {
-                // read the counters (the next level's count, the rows moved,
-                // the tiers' list sizes) while the scatter runs
-                cudaMemcpyAsync(ctx->h_small + 16, ctr, kCtrWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-                cudaEventRecord(ctx->ev_level, s);
-            }
             {
                 LaunchScope ls_(ctx, "msd_scatter");
+                const uint32_t seq = read_back ? ++ctx->read_backs : 0u;
                 launch_k(msd_scatter_kernel<K, RANK, IT>, scatter_grid, kNtM, msd_smem, s, b, lr, more,
-                         (uint32_t)levels);
+                         (uint32_t)levels, read_back ? ctx->h_small : (uint32_t *)nullptr, seq);
+                FMCS_LAUNCH_CHECK("msd level");
                 if (read_back) {
-                    cudaError_t e = cudaEventSynchronize(ctx->ev_level);
-                    if (e != cudaSuccess) return cuda_fail(ctx, e, "sort: level event");
+                    if ((rc = wait_counters(ctx, seq, "sort: level counts"))) return rc;
                     // algorithmic bytes: every moved row is read from the level's
                     // source (the round's bank, through the order when there is
                     // one, at level 0; the work buffers after) and written once
-                    const double moved = (double)ctx->h_small[16 + kCtrMoved];
+                    const double moved = (double)hctr[kCtrMoved];
                     const double rd = host_lvl == 0 ? (double)sizeof(K) + (b.ext_order ? 4.0 : 0.0)
                                                     : (double)sizeof(K) + 4.0;
                     ls_.set_units(moved);
@@ -1232,7 +1229,7 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
                 host_lvl = lvl;
                 if ((rc = level(st, 0, !a.fixed_launches))) return rc;
                 if (!a.fixed_launches) {
-                    nlarge = ctx->h_small[16 + kCtrLarge0 + ((uint32_t)(lvl + 1) & 1u)];
+                    nlarge = hctr[kCtrLarge0 + ((uint32_t)(lvl + 1) & 1u)];
                     tiers_known = true;
                 }
             }
@@ -1463,7 +1460,7 @@ int lsd_sort_full_t(fmcs_ctx *ctx, void *keys, uint32_t *vals, uint64_t n, uint3
         }
         { LaunchScope ls_(ctx, "msd_scatter");
             launch_k(msd_scatter_kernel<K, RANK, IT>, sms * msd_ctas_per_sm(IT), kNtM, msd_smem, st, b, lr,
-                     (cudaGraphConditionalHandle)0, 1u);
+                     (cudaGraphConditionalHandle)0, 1u, (uint32_t *)nullptr, 0u);
         }
         FMCS_LAUNCH_CHECK("lsd pass");
     }
