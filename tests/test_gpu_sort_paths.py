@@ -202,3 +202,38 @@ def test_small_segmented_rounds(ctx, n, dtype, bits):
     bank = (rng.integers(0, 1 << 9, size=n, dtype=np.uint64) % np.uint64(7)).astype(dtype)
     _segmented(ctx, sizes, bank, bits, n, want_keys=True)
     _segmented(ctx, [n], bank, bits, n)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 4096, 4099, 20001])
+@pytest.mark.parametrize("bank_bytes", [1, 2, 4, 8])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_stitch_slices(ctx, n, bank_bytes, offset):
+    """Slices of every source width at every place of the bank (inside a word,
+    across its middle, past its end), on and off a 16-byte boundary, rows that
+    do not fill a group of four."""
+    import torch
+    rng = np.random.default_rng(n * 10 + bank_bytes)
+    tt = {1: torch.uint8, 2: torch.int16, 4: torch.int32, 8: torch.int64}
+    nt = {1: np.uint8, 2: np.uint16, 4: np.uint32, 8: np.uint64}
+    for widest in (1, 2, 4, 8):
+        slices, dev = [], []
+        for _ in range(int(rng.integers(1, 8))):
+            b = int(rng.choice([x for x in (1, 2, 4, 8) if x <= widest]))
+            bits = int(rng.integers(1, 8 * b + 1))
+            start = int(rng.integers(1, bits + 1))
+            end = int(rng.integers(start, bits + 1))
+            v = rng.integers(0, (1 << bits) - 1, size=n, dtype=np.uint64, endpoint=True).astype(nt[b])
+            d = torch.zeros(n + 16, dtype=tt[b], device="cuda")
+            raw = torch.from_numpy(v.view({1: np.uint8, 2: np.int16, 4: np.int32, 8: np.int64}[b]))
+            d[offset:offset + n] = raw.cuda()
+            slices.append((v, bits, start, end))
+            dev.append((d[offset:offset + n], bits, start, end))
+        bank = torch.zeros(n, dtype=tt[bank_bytes], device="cuda")
+        torch.cuda.synchronize()
+        ctx.stitch(dev, bank)
+        want = np.zeros(n, np.uint64)
+        for v, bits, start, end in slices:   # shift left by each slice's width, then or it in
+            w = end - start + 1
+            x = (v.astype(np.uint64) >> np.uint64(bits - end)) & np.uint64((1 << w) - 1)
+            want = x if w == 64 else (want << np.uint64(w)) | x
+        assert np.array_equal(bank.cpu().numpy().view(nt[bank_bytes]), want.astype(nt[bank_bytes]))
