@@ -70,7 +70,7 @@ __device__ __forceinline__ void bank_keys(const SmallParams &p, uint32_t b, cons
 }
 
 template <int NT, int IT>
-struct SmallSmem {
+struct alignas(16) SmallSmem {
     OnchipSmem<uint64_t, NT, IT> sort;
     uint16_t run[NT * IT];      // segment of each input position
     uint32_t wsum[NT / 32];
