@@ -131,6 +131,9 @@ struct LevelRefs {
     // level 0 (one segment) was counted before the sort, by the stitch: its
     // chunks' rows and after them their super rows
     const uint32_t *top_hist;
+    // level 0's histogram pass leaves the keys it gathers through the order in
+    // BUF0, beside the order itself: from then on the segments are BUF0's
+    int gathered;
 };
 
 // The first super row of segment s, whose first chunk is c0.  (Rounding c0
@@ -326,27 +329,59 @@ __global__ void classify_kernel(Bufs<K> b, const uint32_t *__restrict__ seg_star
         }
         return;
     }
-    const uint32_t nseg = seg_start ? *d_nseg : 1u;
-    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x) {
-        const uint32_t start = seg_start ? seg_start[s] : 0u;
-        const uint32_t end = seg_start ? seg_start[s + 1] : (uint32_t)n;
-        const uint32_t len = end - start;
-        if (len == 1) {
-            // A one-row segment keeps its position.  With skip_single its oid
-            // is in BUF0 already and nothing reads its key: nothing to do.
-            // (Fetching those keys was a random 32-byte sector per row: 1.25 ms
-            // of the second round of a 67M-row plan whose first round leaves
-            // one-row groups, against 0.06 ms for reading the segment starts.)
-            if (skip_single) continue;
-            // Otherwise copy it straight to BUF0.
-            K k;
-            uint32_t v;
-            load_kv(b, kSrcExt, start, k, v);
-            b.k0[start] = k;
-            b.v0[start] = v;
-            continue;
+    if (!seg_start) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            if (n == 1) {
+                K k;
+                uint32_t v;
+                load_kv(b, kSrcExt, 0, k, v);
+                b.k0[0] = k;
+                b.v0[0] = v;
+            } else {
+                route_segment(0u, (uint32_t)n, key_bits, kSrcExt, ctr, kCtrLarge0, large0, lists);
+            }
         }
-        route_segment(start, len, key_bits, kSrcExt, ctr, kCtrLarge0, large0, lists);
+        return;
+    }
+    // Four segments a thread, their starts in one 16-byte load (seg_start is
+    // 16-byte aligned): where most segments are one row (a round after nearly
+    // unique keys) this kernel only streams the starts.  67M of them: 126 us one
+    // segment a thread, 57 now.
+    const uint32_t nseg = *d_nseg;
+    const uint32_t stride = gridDim.x * blockDim.x * 4;
+    for (uint64_t s0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4ull; s0 < nseg; s0 += stride) {
+        uint32_t at[5];
+        const uint32_t m = (uint32_t)min((uint64_t)4, nseg - s0);
+        if (m == 4) {
+            const uint4 w = *reinterpret_cast<const uint4 *>(seg_start + s0);
+            at[0] = w.x; at[1] = w.y; at[2] = w.z; at[3] = w.w;
+            at[4] = seg_start[s0 + 4];
+            if (skip_single && at[4] - at[0] == 4) continue;   // four one-row segments
+        } else {
+#pragma unroll
+            for (uint32_t k = 0; k < 5; ++k) at[k] = k <= m ? seg_start[s0 + k] : 0u;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            if (k >= m) break;
+            const uint32_t start = at[k], len = at[k + 1] - at[k];
+            if (len == 1) {
+                // A one-row segment keeps its position.  With skip_single its
+                // oid is in BUF0 already and nothing reads its key: nothing to
+                // do.  (Fetching those keys was a random 32-byte sector per
+                // row: 1.25 ms of the second round of a 67M-row plan whose
+                // first round leaves one-row groups.)
+                if (skip_single) continue;
+                // Otherwise copy it straight to BUF0.
+                K key;
+                uint32_t v;
+                load_kv(b, kSrcExt, start, key, v);
+                b.k0[start] = key;
+                b.v0[start] = v;
+                continue;
+            }
+            route_segment(start, len, key_bits, kSrcExt, ctr, kCtrLarge0, large0, lists);
+        }
     }
 }
 
@@ -482,6 +517,17 @@ __global__ void __launch_bounds__(kNtM, kHistCtas) msd_hist_kernel(Bufs<K> b, Le
                 const uint32_t i = beg + threadIdx.x + j * kNtM;
                 key[j] = i < end ? b.ext_bank[v[j]] : K(0);
             }
+            if (r.gathered) {
+                // the scatter reads them in order instead of gathering again
+                // (32 bytes fetched a row): 60M rows in 64 groups, two rounds,
+                // 3.23 -> 2.54 ms
+                K *kd = b.k0 + sg.start;
+#pragma unroll
+                for (int j = 0; j < MAXJ; ++j) {
+                    const uint32_t i = beg + threadIdx.x + j * kNtM;
+                    if (i < end) kd[i] = key[j];
+                }
+            }
         } else {
             const K *ks = (sg.src == kSrcExt ? b.ext_bank : sg.src == kSrcBuf1 ? b.k1 : b.k0) + sg.start;
 #pragma unroll
@@ -615,7 +661,8 @@ __global__ void __launch_bounds__(kPlanThreads) msd_plan_kernel(LevelRefs r, Lis
         __syncthreads();
     }
     for (uint32_t s = blockIdx.x; s < nseg; s += gridDim.x) {
-        const LargeSeg sg = segs[s];
+        LargeSeg sg = segs[s];
+        if (lvl == 0 && r.gathered) sg.src = kSrcBuf0;
         const uint32_t r0 = r.chunk_prefix[s], r1 = r.chunk_prefix[s + 1];
         const uint32_t s0 = top ? 0u : super_row(r0, s);
         const uint32_t tot = sum_rows(super, s0, s0 + (r1 - r0 - 1) / kSuper + 1);
@@ -1125,6 +1172,7 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
     lr.ctr = ctr;
     lr.dev_level = 1;
     lr.top_hist = a.seg_start ? nullptr : a.top_hist;
+    lr.gathered = a.order_in && a.order_in == a.order_out;
 
     const int sms = ctx->num_sms;
     // classification of the initial segments
