@@ -75,52 +75,80 @@ int counters(fmcs_ctx *ctx, uint32_t **w)
     return rc;
 }
 
-// One sort round on device data.  order (device) is in/out; seg_start/d_nseg
-// describe the runs of in_group when the caller already has them.
+// One sort round on device data.  order (device) is in/out; the segments are
+// seg_start / d_nseg (NULL: one segment), the runs of in_group.  The group count,
+// the group ids (out_group) and the next round's segments (next_seg_start) follow
+// from the flags (SortArgs::flags; mark_starts: the segments passed in are not
+// flagged yet; no keys_out then), or without flags from the sorted keys and in_group.
 int sort_round_dev(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, uint32_t key_bits, uint32_t *order,
-                   const uint32_t *in_group, const uint32_t *seg_start, const uint32_t *d_nseg,
-                   uint32_t *out_group, void *keys_out, uint32_t *next_seg_start, uint32_t *d_next_nseg,
-                   uint64_t n, uint32_t *d_ngroups, bool identity_order = false, bool fixed_launches = false,
+                   const uint32_t *in_group, const uint32_t *seg_start, const uint32_t *d_nseg, uint8_t *flags,
+                   bool mark_starts, uint32_t *out_group, void *keys_out, uint32_t *next_seg_start, uint32_t *d_count,
+                   uint64_t n, bool identity_order = false, bool fixed_launches = false,
                    const uint32_t *top_hist = nullptr)
 {
     int rc;
     void *p;
-    // The keys of one-row segments are not needed when only the boundary scan
-    // below reads them: such a row and the row after it start a group whatever
-    // their keys, because in_group differs there.
-    const bool keys_scratch = !keys_out && in_group;
+    SortArgs a;
+    // nobody reads the key of a one-row segment: the scan below starts a group at
+    // such a row and at the row after it whatever their keys (in_group differs)
+    a.skip_single = !keys_out && seg_start;
     if (!keys_out) {
         if ((rc = ws_get(ctx, kSlotKeys0, n * bank_bytes, &p))) return rc;
         keys_out = p;
     }
-    uint32_t *w;
-    if ((rc = counters(ctx, &w))) return rc;
-    if (in_group && !seg_start) {
-        if ((rc = ws_get(ctx, kSlotSegStart, (n + 2) * sizeof(uint32_t), &p))) return rc;
-        uint32_t *ss = (uint32_t *)p;
-        if ((rc = launch_segments(ctx, in_group, ss, w + kCtrNgroups + 1, n))) return rc;
-        seg_start = ss;
-        d_nseg = w + kCtrNgroups + 1;
-    }
-    SortArgs a;
     a.bank = bank;
     a.bank_bytes = bank_bytes;
     a.key_bits = key_bits;
-    a.order_in = (in_group && !identity_order) ? order : nullptr;
-    a.seg_start = in_group ? seg_start : nullptr;
+    a.order_in = (seg_start && !identity_order) ? order : nullptr;
+    a.seg_start = seg_start;
     a.nseg_host = 0;
-    a.d_nseg = in_group ? d_nseg : nullptr;
+    a.d_nseg = d_nseg;
     a.order_out = order;
     a.keys_out = keys_out;
     a.n = n;
     a.fixed_launches = fixed_launches;
-    a.top_hist = in_group ? nullptr : top_hist;
-    a.keys_scratch = keys_scratch;
+    a.top_hist = seg_start ? nullptr : top_hist;
+    a.flags = flags;
+    a.mark_starts = mark_starts;
     if ((rc = sort_segments(ctx, a))) return rc;
+    if (flags) return launch_flag_rank(ctx, flags, out_group, n, d_count, next_seg_start);
     if (out_group || next_seg_start)
-        return launch_group_ids_segments(ctx, keys_out, bank_bytes, in_group, out_group, next_seg_start, n,
-                                         next_seg_start ? d_next_nseg : d_ngroups);
+        return launch_group_ids_segments(ctx, keys_out, bank_bytes, in_group, out_group, next_seg_start, n, d_count);
     return FMCS_OK;
+}
+
+// Plans of fewer rows than this find their groups by a scan of the sorted keys:
+// flags save 14 bytes a row of traffic (8-byte keys) and cost the on-chip sorts
+// some instructions and a store.  16.8M rows [50] 634 us by keys, 621 by flags;
+// 384 instances (38.6M rows) 2.78 and 2.68 ms; but 90,001 rows 174 and 183.
+constexpr uint64_t kFlagRows = 1ull << 20;
+
+// The group-start flags of n rows (every sort round writes what it splits).
+int flags_of(fmcs_ctx *ctx, uint64_t n, uint8_t **flags)
+{
+    void *p;
+    const int rc = ws_get(ctx, kSlotFlags, n, &p);
+    *flags = (uint8_t *)p;
+    return rc;
+}
+
+// fmcs_sort_round over more rows than one launch takes: the segments come from
+// in_group.
+int sort_round_large(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, uint32_t key_bits, uint32_t *order,
+                     const uint32_t *in_group, uint32_t *out_group, void *keys_out, uint64_t n, uint32_t *d_ng)
+{
+    int rc;
+    void *p;
+    uint32_t *w;
+    if ((rc = counters(ctx, &w))) return rc;
+    uint32_t *seg_start = nullptr, *d_nseg = w + kCtrNgroups + 1;
+    if (in_group) {
+        if ((rc = ws_get(ctx, kSlotSegStart, (n + 2) * sizeof(uint32_t), &p))) return rc;
+        seg_start = (uint32_t *)p;
+        if ((rc = launch_segments(ctx, in_group, seg_start, d_nseg, n))) return rc;
+    }
+    return sort_round_dev(ctx, bank, bank_bytes, key_bits, order, in_group, seg_start, seg_start ? d_nseg : nullptr,
+                          nullptr, false, out_group, keys_out, nullptr, d_ng, n);
 }
 
 // The device work of one plan (stitch + rounds), enqueued on the context's
@@ -151,15 +179,21 @@ int plan_pipeline(fmcs_ctx *ctx, const Plan &plan, const void *const *dcols, con
             return launch_small_plan(ctx, sl.data(), ns.data(), nbanks, n, dorder, dgroup_out, d_ng);
         }
     }
-    // group ping-pong and segment starts
-    uint32_t *g[2];
-    if ((rc = ws_get(ctx, kSlotGroupA, n * 4, &p))) return rc;
-    g[0] = (uint32_t *)p;
-    if ((rc = ws_get(ctx, kSlotGroupB, n * 4, &p))) return rc;
-    g[1] = (uint32_t *)p;
-    uint32_t *segs[2];
-    if ((rc = ws_get(ctx, kSlotSegStart, 2 * carve_round((n + 2) * sizeof(uint32_t)), &p))) return rc;
-    {
+    // group ping-pong (hash rounds, and sort rounds without flags), flags, and
+    // segment starts
+    uint32_t *g[2] = {nullptr, nullptr};
+    uint32_t *segs[2] = {nullptr, nullptr};
+    uint8_t *flags = nullptr;
+    if (!hash && n >= kFlagRows) {
+        if ((rc = flags_of(ctx, n, &flags))) return rc;
+    } else {
+        if ((rc = ws_get(ctx, kSlotGroupA, n * 4, &p))) return rc;
+        g[0] = (uint32_t *)p;
+        if ((rc = ws_get(ctx, kSlotGroupB, n * 4, &p))) return rc;
+        g[1] = (uint32_t *)p;
+    }
+    if (!hash && nbanks > 1) {
+        if ((rc = ws_get(ctx, kSlotSegStart, 2 * carve_round((n + 2) * sizeof(uint32_t)), &p))) return rc;
         Carver cv(p);
         segs[0] = cv.take<uint32_t>(n + 2);
         segs[1] = cv.take<uint32_t>(n + 2);
@@ -214,12 +248,13 @@ int plan_pipeline(fmcs_ctx *ctx, const Plan &plan, const void *const *dcols, con
             if ((rc = stitch_bank(b + 1, ctx->par, &next_bank))) return rc;
         }
         if (b > 0) top_hist = nullptr;
-        uint32_t *og = last ? (uint32_t *)(dgroup_out ? dgroup_out : g[b & 1]) : g[b & 1];
+        uint32_t *og = last && dgroup_out ? dgroup_out : g[b & 1];
         if (!hash) {
-            // (b)+(d): sort, then group ids (+ the next round's segments)
+            // (b)+(d): sort, then group ids (last round) or the next round's segments
             uint32_t *ns = last ? nullptr : segs[b & 1];
-            if ((rc = sort_round_dev(ctx, bank, bp.bytes, bp.bits, dorder, in_group, seg_in, d_nseg_in, og, nullptr,
-                                     ns, d_nseg[b & 1], n, d_ng, false, fixed, top_hist)))
+            if ((rc = sort_round_dev(ctx, bank, bp.bytes, bp.bits, dorder, in_group, seg_in, d_nseg_in, flags, false,
+                                     flags && !last ? nullptr : og, nullptr, ns, last ? d_ng : d_nseg[b & 1], n, false,
+                                     fixed, top_hist)))
                 return rc;
             seg_in = ns;
             d_nseg_in = d_nseg[b & 1];
@@ -386,8 +421,8 @@ extern "C" int fmcs_sort_round(fmcs_ctx *ctx, const void *bank, uint32_t bank_by
         rc = launch_small_round(ctx, dbank, bank_bytes, key_bits, dig ? (const uint32_t *)dorder : nullptr,
                                 (const uint32_t *)dig, (uint32_t *)dorder, (uint32_t *)dgroup, dkeys, n, d_ng);
     else
-        rc = sort_round_dev(ctx, dbank, bank_bytes, key_bits, (uint32_t *)dorder, (const uint32_t *)dig, nullptr,
-                            nullptr, (uint32_t *)dgroup, dkeys, nullptr, nullptr, n, d_ng);
+        rc = sort_round_large(ctx, dbank, bank_bytes, key_bits, (uint32_t *)dorder, (const uint32_t *)dig,
+                              (uint32_t *)dgroup, dkeys, n, d_ng);
     if (rc) return rc;
     if (h_order && (rc = copy_out(ctx, order, dorder, n * 4))) return rc;
     if (h_group && (rc = copy_out(ctx, out_group, dgroup, n * 4))) return rc;
@@ -620,11 +655,10 @@ extern "C" int fmcs_run_plan_desc(fmcs_ctx *ctx, const void *const *cols, const 
 namespace fmcs {
 namespace {
 
-// The two kernels over all rows of a batch take 8,192 consecutive rows a CTA
-// step: a warp finds the instances of the step's first and last row, and a row
-// is searched for between those two only (mostly the same one).  Reading an
-// id per row, or searching for it among all instances, cost 288 and 438 us for
-// 38.6M rows; the bytes moved (4 and 16 a row) take 24 and 95.
+// The kernel over all rows of a batch takes 8,192 consecutive rows a CTA step: a
+// warp finds the instances of the step's first and last row, and a row is
+// searched for between those two only (mostly the same one).  Reading an id per
+// row cost 438 us for 38.6M rows, this 164; the 16 bytes a row take 95.
 constexpr uint32_t kInstRows = 8192;
 
 __device__ __forceinline__ uint32_t instance_of(const uint32_t *starts, uint32_t lo, uint32_t hi, uint32_t i)
@@ -634,30 +668,6 @@ __device__ __forceinline__ uint32_t instance_of(const uint32_t *starts, uint32_t
         if (starts[mid] <= i) lo = mid; else hi = mid - 1;
     }
     return lo;
-}
-
-__global__ void __launch_bounds__(256) instance_ids_kernel(const uint32_t *__restrict__ starts, uint32_t ninst,
-                                                           uint32_t *__restrict__ inst_id, uint64_t n)
-{
-    kernel_prologue();
-    for (uint64_t base = blockIdx.x * (uint64_t)kInstRows; base < n; base += (uint64_t)gridDim.x * kInstRows) {
-        const uint64_t end = min(n, base + kInstRows);
-        const uint32_t lo = find_segment_warp(starts, ninst, (uint32_t)base);
-        const uint32_t hi = find_segment_warp(starts, ninst, (uint32_t)(end - 1));
-        for (uint64_t i = base + threadIdx.x * 4; i < end; i += blockDim.x * 4) {
-            uint32_t k = instance_of(starts, lo, hi, (uint32_t)i), v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                while (k < hi && starts[k + 1] <= i + j) ++k;
-                v[j] = k;
-            }
-            if (i + 4 <= n) {   // (inst_id starts on a 256-byte boundary)
-                *reinterpret_cast<uint4 *>(inst_id + i) = make_uint4(v[0], v[1], v[2], v[3]);
-            } else {
-                for (int j = 0; j < 4 && i + j < n; ++j) inst_id[i + j] = v[j];
-            }
-        }
-    }
 }
 
 __global__ void instance_bases_kernel(const uint32_t *starts, uint32_t ninst, const uint32_t *group, uint32_t *base,
@@ -755,20 +765,15 @@ extern "C" int fmcs_run_batch(fmcs_ctx *ctx, const void *const *cols, const uint
     // instance starts, ids per row, bases and counts
     if ((rc = ws_get(ctx, kSlotMisc,
                      carve_total({(ninst + 1) * sizeof(uint32_t), ninst * sizeof(uint32_t),
-                                  (ninst + 1) * sizeof(uint32_t), n * sizeof(uint32_t)}),
+                                  (ninst + 1) * sizeof(uint32_t)}),
                      &p)))
         return rc;
     Carver cv(p);
     uint32_t *d_starts = cv.take<uint32_t>(ninst + 1);
     uint32_t *d_base = cv.take<uint32_t>(ninst);
     uint32_t *d_count = cv.take<uint32_t>(ninst + 1);
-    uint32_t *inst_id = cv.take<uint32_t>(n);
     cudaError_t e = cudaMemcpyAsync(d_starts, starts.data(), (ninst + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "fmcs_run_batch upload");
-    {
-        LaunchScope ls_(ctx, "instance_ids");
-        launch_k(instance_ids_kernel, ctx->num_sms * 8, 256, 0, st, (const uint32_t *)d_starts, ninst, inst_id, n);
-    }
     uint32_t *w;
     if ((rc = counters(ctx, &w))) return rc;
     uint32_t *d_ng = w + kCtrNgroups;
@@ -799,21 +804,22 @@ extern "C" int fmcs_run_batch(fmcs_ctx *ctx, const void *const *cols, const uint
     bool h_order, h_group;
     if ((rc = stage_out(ctx, order_out, n * 4, kSlotStageOut0, &dorder, &h_order))) return rc;
     if ((rc = stage_out(ctx, group_out, n * 4, kSlotStageOut1, &dgroup_out, &h_group))) return rc;
-    uint32_t *g[2];
-    if ((rc = ws_get(ctx, kSlotGroupA, n * 4, &p))) return rc;
-    g[0] = (uint32_t *)p;
-    if ((rc = ws_get(ctx, kSlotGroupB, n * 4, &p))) return rc;
-    g[1] = (uint32_t *)p;
-    uint32_t *segs[2];
-    if ((rc = ws_get(ctx, kSlotSegStart, 2 * carve_round((n + 2) * sizeof(uint32_t)), &p))) return rc;
-    {
+    uint32_t *group = (uint32_t *)dgroup_out;   // the last round's group ids
+    if (!group) {
+        if ((rc = ws_get(ctx, kSlotGroupA, n * 4, &p))) return rc;
+        group = (uint32_t *)p;
+    }
+    uint32_t *segs[2] = {nullptr, nullptr};
+    if (nbanks > 1) {
+        if ((rc = ws_get(ctx, kSlotSegStart, 2 * carve_round((n + 2) * sizeof(uint32_t)), &p))) return rc;
         Carver cv(p);
         segs[0] = cv.take<uint32_t>(n + 2);
         segs[1] = cv.take<uint32_t>(n + 2);
     }
+    uint8_t *flags;
+    if ((rc = flags_of(ctx, n, &flags))) return rc;
     uint32_t *d_nseg[2] = {w + kCtrNgroups + 2, w + kCtrNgroups + 3};
-    // round 0 is segmented by instance: instance ids are the incoming groups
-    const uint32_t *in_group = inst_id;
+    // round 0 is segmented by instance (its starts are flagged by that round)
     const uint32_t *seg_in = d_starts;
     const uint32_t *d_nseg_in = d_ninst;
     // (as in a single plan, the next round's bank is stitched on the second
@@ -846,26 +852,24 @@ extern "C" int fmcs_run_batch(fmcs_ctx *ctx, const void *const *cols, const uint
             if ((rc = fork_par(ctx, ctx->stream))) return rc;
             if ((rc = stitch_bank(b + 1, ctx->par, &next_bank))) return rc;
         }
-        uint32_t *og = (last && dgroup_out) ? (uint32_t *)dgroup_out : g[b & 1];
         uint32_t *ns = last ? nullptr : segs[b & 1];
-        if ((rc = sort_round_dev(ctx, bank, bp.bytes, bp.bits, (uint32_t *)dorder, in_group, seg_in, d_nseg_in, og,
-                                 nullptr, ns, d_nseg[b & 1], n, d_ng, b == 0)))
+        if ((rc = sort_round_dev(ctx, bank, bp.bytes, bp.bits, (uint32_t *)dorder, nullptr, seg_in, d_nseg_in, flags, b == 0,
+                                 last ? group : nullptr, nullptr, ns, last ? d_ng : d_nseg[b & 1], n, b == 0)))
             return rc;
         seg_in = ns;
         d_nseg_in = d_nseg[b & 1];
-        in_group = og;
     }
     ctx->prof_round = -1;
     // instance-local oids and group ids
     {
         LaunchScope ls_(ctx, "instance_bases");
-        launch_k(instance_bases_kernel, (ninst + 255) / 256, 256, 0, st, d_starts, ninst, in_group, d_base, d_count);
+        launch_k(instance_bases_kernel, (ninst + 255) / 256, 256, 0, st, d_starts, ninst, group, d_base, d_count);
     }
     {
         LaunchScope ls_(ctx, "localize");
         launch_k(localize_kernel, ctx->num_sms * 8, 256, 0, st, (const uint32_t *)d_starts, ninst,
-                 (const uint32_t *)d_base, (uint32_t *)dorder, (uint32_t *)in_group, n,
-                 (((uintptr_t)dorder | (uintptr_t)in_group) & 15u) == 0);
+                 (const uint32_t *)d_base, (uint32_t *)dorder, group, n,
+                 (((uintptr_t)dorder | (uintptr_t)group) & 15u) == 0);
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "fmcs_run_batch localize");

@@ -48,6 +48,7 @@ enum Slot : int {
     kSlotGroupA,      // run_plan group ping
     kSlotGroupB,      // run_plan group pong
     kSlotColStage,    // run_plan host column staging (several columns)
+    kSlotFlags,       // group-start flags of a plan's rows
     kSlotTopHist,     // level-0 digit histogram of a round-0 bank, counted by the stitch
     kSlotMisc,
     kSlotCount
@@ -249,9 +250,13 @@ struct SortArgs {
     // says the rows are in order already (every segment is only copied).
     const uint32_t *d_key_bits = nullptr;
     const uint32_t *d_in_order = nullptr;
-    // The caller uses keys_out only to find the boundaries inside the segments
-    // it passed in: the key of a one-row segment need not be written.
-    bool keys_scratch = false;
+    // flags (n bytes, or NULL): 1 where a group of equal keys starts inside its
+    // segment or a segment starts, 0 elsewhere.  Written for every row but those
+    // of one-row segments passed in: their flags are the round before's, unless
+    // mark_starts has them written, too.  keys_out is scratch then.
+    uint8_t *flags = nullptr;
+    bool mark_starts = false;
+    bool skip_single = false;   // (without flags, too) the keys of one-row segments need not be written
 };
 int sort_segments(fmcs_ctx *ctx, const SortArgs &a);
 // Rows per chunk of an HBM radix level of a round of n rows (tiles of the
@@ -292,8 +297,10 @@ int launch_group_ids_segments(fmcs_ctx *ctx, const void *keys, uint32_t key_byte
                               uint32_t *out_group, uint32_t *seg_start, uint64_t n, uint32_t *d_count);
 // v[i] = i
 int launch_iota(fmcs_ctx *ctx, uint32_t *v, uint64_t n);
-// rank[i] = (number of set flags in [0, i]) - 1; *d_count = number of set flags.
-int launch_flag_rank(fmcs_ctx *ctx, const uint8_t *flags, uint32_t *rank, uint64_t n, uint32_t *d_count);
+// rank[i] = (number of set flags in [0, i]) - 1 (rank may be NULL); *d_count =
+// number of set flags; with seg_start, the positions of the set flags and then n.
+int launch_flag_rank(fmcs_ctx *ctx, const uint8_t *flags, uint32_t *rank, uint64_t n, uint32_t *d_count,
+                     uint32_t *seg_start = nullptr);
 
 // ---------------------------------------------------------------- hash grouping
 // fixed_launches: the same launches whatever the data, with no host

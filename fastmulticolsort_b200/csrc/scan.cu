@@ -83,7 +83,8 @@ struct ScanLayout {
     static constexpr bool kGroup = (MODE & kScanGroup) != 0;
     static constexpr bool kFlags = MODE == kScanFlags;
     static constexpr int kKeyBytes = kKeys ? (int)sizeof(K) : 1;
-    static constexpr int kWidest = kFlags ? 1 : (kGroup && kKeyBytes < 4 ? 4 : kKeyBytes);
+    // (flags: 4 a lane and load, so that pass 3's ids are stored 16 bytes a lane)
+    static constexpr int kWidest = kFlags ? 4 : (kGroup && kKeyBytes < 4 ? 4 : kKeyBytes);
     static constexpr int P = 16 / kWidest;
     static constexpr int C = kScanItems / P;
     // per-chunk counts packed into one 64-bit word, in fields wide enough for
@@ -333,6 +334,7 @@ void launch_scan_mode(cudaStream_t st, const K *keys, const uint32_t *in_group, 
     uint32_t *tile_count = tile_work, *tile_prefix = tile_work + tiles;
     launch_k(scan_count_kernel<K, MODE, VEC>, tiles, kScanThreads, 0, st, keys, in_group, flags, n, tile_count, masks);
     launch_k(scan_prefix_kernel, 1, 1024, 0, st, (const uint32_t *)tile_count, tiles, tile_prefix, d_count, seg_start, n);
+    if (!out_group && !seg_start) return;   // only the count was wanted
     if (masks)
         launch_k(scan_ids_kernel<K, MODE, VEC, true>, tiles, kScanThreads, 0, st, keys, in_group, flags, n,
                  (const uint32_t *)tile_prefix, (const uint16_t *)masks, out_group, seg_start);
@@ -451,9 +453,10 @@ int launch_iota(fmcs_ctx *ctx, uint32_t *v, uint64_t n)
     return e == cudaSuccess ? FMCS_OK : cuda_fail(ctx, e, "iota launch");
 }
 
-int launch_flag_rank(fmcs_ctx *ctx, const uint8_t *flags, uint32_t *rank, uint64_t n, uint32_t *d_count)
+int launch_flag_rank(fmcs_ctx *ctx, const uint8_t *flags, uint32_t *rank, uint64_t n, uint32_t *d_count,
+                     uint32_t *seg_start)
 {
-    return run_boundary_scan(ctx, nullptr, 0, nullptr, flags, rank, nullptr, n, d_count);
+    return run_boundary_scan(ctx, nullptr, 0, nullptr, flags, rank, seg_start, n, d_count);
 }
 
 }  // namespace fmcs

@@ -162,6 +162,12 @@ struct Bufs {
     uint32_t *v0, *v1;
     const K *ext_bank;
     const uint32_t *ext_order;   // NULL: iota
+    // Per row, in the sorted order: 1 where its key differs from the row before
+    // in its segment, or a segment starts (NULL: not wanted).  Whoever puts a
+    // segment in its final order writes them, with the keys at hand: the group
+    // ids then read a byte a row, and the sorted keys are not written.
+    uint8_t *flags;
+    int write_keys;   // 1 without flags
 };
 
 template <typename K>
@@ -236,6 +242,7 @@ struct Lists {
     LargeSeg *copy;        // segments that only need to reach BUF0, <= kCopySplit rows (warp each)
     LargeSeg *copy_large;  // the same, larger: copied by tiles across the grid
     uint32_t local_max;   // segments above this size take the MSD levels (tuned, <= kCapLocal)
+    uint8_t *flags;       // Bufs::flags
 };
 
 // Route a segment (child or initial) to its tier.  Segments that need no
@@ -260,7 +267,9 @@ __device__ __forceinline__ int route_segment(uint32_t start, uint32_t len, uint3
     if (len == 0) return -1;
     int which;
     if (len == 1 || shift == 0) {
-        if (src == kSrcBuf0) return -1;   // already in place
+        if (L.flags) L.flags[start] = 1;
+        // already in place (with flags, the copy kernels still write its other rows')
+        if (src == kSrcBuf0 && (len == 1 || !L.flags)) return -1;
         which = len > kCopySplit ? kCtrCopyLarge : kCtrCopy;
     } else if (len > L.local_max) {
         which = large_ctr;
@@ -314,7 +323,7 @@ template <typename K>
 __global__ void classify_kernel(Bufs<K> b, const uint32_t *__restrict__ seg_start, const uint32_t *d_nseg,
                                 uint64_t n, uint32_t key_bits, uint32_t *ctr, LargeSeg *large0, Lists lists,
                                 const uint32_t *top_hist, const uint32_t *d_key_bits,
-                                const uint32_t *d_in_order, bool skip_single)
+                                const uint32_t *d_in_order, bool skip_single, bool mark_starts)
 {
     kernel_prologue();
     if (d_key_bits) key_bits = min(key_bits, *d_key_bits);
@@ -337,6 +346,7 @@ __global__ void classify_kernel(Bufs<K> b, const uint32_t *__restrict__ seg_star
                 load_kv(b, kSrcExt, 0, k, v);
                 b.k0[0] = k;
                 b.v0[0] = v;
+                if (b.flags) b.flags[0] = 1;
             } else {
                 route_segment(0u, (uint32_t)n, key_bits, kSrcExt, ctr, kCtrLarge0, large0, lists);
             }
@@ -356,7 +366,13 @@ __global__ void classify_kernel(Bufs<K> b, const uint32_t *__restrict__ seg_star
             const uint4 w = *reinterpret_cast<const uint4 *>(seg_start + s0);
             at[0] = w.x; at[1] = w.y; at[2] = w.z; at[3] = w.w;
             at[4] = seg_start[s0 + 4];
-            if (skip_single && at[4] - at[0] == 4) continue;   // four one-row segments
+            if (skip_single && at[1] - at[0] == 1 && at[2] - at[1] == 1 && at[3] - at[2] == 1 && at[4] - at[3] == 1) {
+                if (mark_starts) {
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k) b.flags[at[0] + k] = 1;
+                }
+                continue;
+            }
         } else {
 #pragma unroll
             for (uint32_t k = 0; k < 5; ++k) at[k] = k <= m ? seg_start[s0 + k] : 0u;
@@ -365,6 +381,7 @@ __global__ void classify_kernel(Bufs<K> b, const uint32_t *__restrict__ seg_star
         for (uint32_t k = 0; k < 4; ++k) {
             if (k >= m) break;
             const uint32_t start = at[k], len = at[k + 1] - at[k];
+            if (mark_starts && len) b.flags[start] = 1;
             if (len == 1) {
                 // A one-row segment keeps its position.  With skip_single its
                 // oid is in BUF0 already and nothing reads its key: nothing to
@@ -376,7 +393,7 @@ __global__ void classify_kernel(Bufs<K> b, const uint32_t *__restrict__ seg_star
                 K key;
                 uint32_t v;
                 load_kv(b, kSrcExt, start, key, v);
-                b.k0[start] = key;
+                if (b.write_keys) b.k0[start] = key;
                 b.v0[start] = v;
                 continue;
             }
@@ -867,7 +884,8 @@ __global__ void __launch_bounds__(kNtM, msd_ctas_per_sm(IT)) msd_scatter_kernel(
 // local tiers
 // ---------------------------------------------------------------------------
 // One segment, on chip (onchip.cuh): one HBM read and one write per row.
-template <typename K, int NT, int IT>
+// FLAGS: it writes the rows' flags, otherwise their keys.
+template <typename K, int NT, int IT, bool FLAGS>
 __device__ __forceinline__ void onchip_sort(OnchipSmem<K, NT, IT> &sm, const Bufs<K> &b, uint32_t start, uint32_t len,
                                             uint32_t src)
 {
@@ -892,31 +910,46 @@ __device__ __forceinline__ void onchip_sort(OnchipSmem<K, NT, IT> &sm, const Buf
     const OnchipInfo f = onchip_core<K, NT, IT>(sm, c, steps, wbase, len);
     K *ko = b.k0 + start;
     uint32_t *vo = b.v0 + start;
+    uint8_t *fo = b.flags + start;
     if (f.same) {
-        if (src != kSrcBuf0) {
 #pragma unroll
-            for (int j = 0; j < IT; ++j) {
-                const uint32_t p = wbase + j * 32 + lane;
-                if (j < (int)steps && p < len) {
-                    ko[p] = (K)c[j];
+        for (int j = 0; j < IT; ++j) {
+            const uint32_t p = wbase + j * 32 + lane;
+            if (j < (int)steps && p < len) {
+                if (src != kSrcBuf0) {
+                    if (!FLAGS) ko[p] = (K)c[j];
                     vo[p] = sm.vals[p];
                 }
+                if (FLAGS) fo[p] = p == 0;
             }
         }
     } else {
         // every load of this segment is done (the sort's barriers) before the
         // first store into BUF0, which may alias the EXT oids of the range
+        const uint32_t pmask = (1u << f.nbits) - 1u;
         for (uint32_t p = tid; p < len; p += NT) {
-            uint32_t q;
-            ko[p] = (K)onchip_key(sm, f, sm.cs[p], &q);
+            const unsigned long long x = sm.cs[p];
+            const uint32_t q = (uint32_t)x & pmask;
             vo[p] = sm.vals[q];
+            if (!FLAGS) {
+                uint32_t q_;
+                ko[p] = (K)onchip_key(sm, f, x, &q_);
+            }
+            if (FLAGS) {
+                const unsigned long long y = sm.cs[p ? p - 1 : 0u];
+                bool differs = p == 0 || (x ^ y) > pmask;
+                if constexpr (sizeof(K) == 8) {
+                    if (f.drop && !differs) differs = sm.lo[q] != sm.lo[(uint32_t)y & pmask];
+                }
+                fo[p] = differs;
+            }
         }
     }
     group_sync<NT>();
 }
 
 // CTA per segment.  1024 threads per SM for every tier (64 registers a thread).
-template <typename K, int NT, int IT>
+template <typename K, int NT, int IT, bool FLAGS>
 __global__ void __launch_bounds__(NT, 1024 / NT)
 block_sort_kernel(Bufs<K> b, const uint2 *list, const uint32_t *d_count)
 {
@@ -925,7 +958,7 @@ block_sort_kernel(Bufs<K> b, const uint2 *list, const uint32_t *d_count)
     const uint32_t count = *d_count;
     for (uint32_t e = blockIdx.x; e < count; e += gridDim.x) {
         const uint2 ent = list[e];
-        onchip_sort<K, NT, IT>(*reinterpret_cast<OnchipSmem<K, NT, IT> *>(smem_raw), b, ent.x, ent.y & 0xFFFFu,
+        onchip_sort<K, NT, IT, FLAGS>(*reinterpret_cast<OnchipSmem<K, NT, IT> *>(smem_raw), b, ent.x, ent.y & 0xFFFFu,
                                (ent.y >> 24) & 3u);
     }
 }
@@ -933,7 +966,7 @@ block_sort_kernel(Bufs<K> b, const uint2 *list, const uint32_t *d_count)
 // Warp per segment, kWarpsA warps a CTA.  The grid is what fits at once.
 constexpr int kWarpsA = 4;
 constexpr int warp_ctas_per_sm(int it) { return it <= 4 ? 10 : 7; }
-template <typename K, int IT>
+template <typename K, int IT, bool FLAGS>
 __global__ void __launch_bounds__(kWarpsA * 32, warp_ctas_per_sm(IT))
 warp_sort_kernel(Bufs<K> b, const uint2 *list, const uint32_t *d_count)
 {
@@ -943,7 +976,7 @@ warp_sort_kernel(Bufs<K> b, const uint2 *list, const uint32_t *d_count)
     const uint32_t count = *d_count;
     for (uint32_t e = blockIdx.x * kWarpsA + (threadIdx.x >> 5); e < count; e += gridDim.x * kWarpsA) {
         const uint2 ent = list[e];
-        onchip_sort<K, 32, IT>(sm, b, ent.x, ent.y & 0xFFFFu, (ent.y >> 24) & 3u);
+        onchip_sort<K, 32, IT, FLAGS>(sm, b, ent.x, ent.y & 0xFFFFu, (ent.y >> 24) & 3u);
     }
 }
 
@@ -951,7 +984,7 @@ warp_sort_kernel(Bufs<K> b, const uint2 *list, const uint32_t *d_count)
 // registers and an odd-even transposition network of N rounds sorts them.
 // It swaps only strictly inverted neighbours, so equal keys keep their order
 // (stable); the padding slots hold the largest key and stay behind the rows.
-template <typename K, int N>
+template <typename K, int N, bool FLAGS>
 __device__ __forceinline__ void sort_tiny(const Bufs<K> &b, uint32_t start, uint32_t len, uint32_t src)
 {
     K k[N];
@@ -979,13 +1012,14 @@ __device__ __forceinline__ void sort_tiny(const Bufs<K> &b, uint32_t start, uint
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         if (i < (int)len) {
-            b.k0[(uint64_t)start + i] = k[i];
+            if (!FLAGS) b.k0[(uint64_t)start + i] = k[i];
             b.v0[(uint64_t)start + i] = v[i];
+            if (FLAGS) b.flags[(uint64_t)start + i] = i == 0 || k[i] != k[i > 0 ? i - 1 : 0];
         }
     }
 }
 
-template <typename K, int NMAX>
+template <typename K, int NMAX, bool FLAGS>
 __global__ void __launch_bounds__(256) thread_sort_kernel(Bufs<K> b, const uint2 *list, const uint32_t *d_count)
 {
     kernel_prologue();
@@ -996,17 +1030,33 @@ __global__ void __launch_bounds__(256) thread_sort_kernel(Bufs<K> b, const uint2
         const uint32_t len = ent.y & 0xFFFFu;
         const uint32_t src = (ent.y >> 24) & 3u;
         if constexpr (NMAX > 16) {
-            sort_tiny<K, NMAX>(b, start, len, src);
+            sort_tiny<K, NMAX, FLAGS>(b, start, len, src);
         } else {
-            if (len <= 2) sort_tiny<K, 2>(b, start, len, src);
-            else if (len <= 4) sort_tiny<K, 4>(b, start, len, src);
-            else if (len <= 8) sort_tiny<K, 8>(b, start, len, src);
-            else sort_tiny<K, 16>(b, start, len, src);
+            if (len <= 2) sort_tiny<K, 2, FLAGS>(b, start, len, src);
+            else if (len <= 4) sort_tiny<K, 4, FLAGS>(b, start, len, src);
+            else if (len <= 8) sort_tiny<K, 8, FLAGS>(b, start, len, src);
+            else sort_tiny<K, 16, FLAGS>(b, start, len, src);
         }
     }
 }
 
-// Segments that need no sorting but sit outside BUF0: one warp per entry.
+// A row of a segment that needs no sorting: to BUF0 unless it is there, and its
+// flag (the segment's keys are equal).
+template <typename K>
+__device__ __forceinline__ void copy_row(const Bufs<K> &b, const LargeSeg &sg, uint64_t r)
+{
+    if ((sg.src & 3u) != kSrcBuf0) {
+        K k;
+        uint32_t v;
+        load_kv(b, sg.src & 3u, r, k, v);
+        if (b.write_keys) b.k0[r] = k;
+        b.v0[r] = v;
+    }
+    if (b.flags) b.flags[r] = r == sg.start;
+}
+
+// Segments that need no sorting but sit outside BUF0 (or lack their flags): one
+// warp per entry.
 template <typename K>
 __global__ void __launch_bounds__(256) copy_kernel(Bufs<K> b, const LargeSeg *list, const uint32_t *d_count)
 {
@@ -1016,14 +1066,7 @@ __global__ void __launch_bounds__(256) copy_kernel(Bufs<K> b, const LargeSeg *li
     const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
     for (uint32_t e = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); e < count; e += nwarps) {
         const LargeSeg sg = list[e];
-        for (uint32_t i = lane; i < sg.len; i += 32) {
-            const uint64_t r = (uint64_t)sg.start + i;
-            K k;
-            uint32_t v;
-            load_kv(b, sg.src & 3u, r, k, v);
-            b.k0[r] = k;
-            b.v0[r] = v;
-        }
+        for (uint32_t i = lane; i < sg.len; i += 32) copy_row(b, sg, (uint64_t)sg.start + i);
     }
 }
 
@@ -1042,13 +1085,7 @@ __global__ void __launch_bounds__(256) copy_tiles_kernel(Bufs<K> b, const LargeS
         const LargeSeg sg = list[s];
         const uint64_t beg = (uint64_t)sg.start + (uint64_t)(t - tile_prefix[s]) * kCopySplit;
         const uint64_t end = min((uint64_t)sg.start + sg.len, beg + kCopySplit);
-        for (uint64_t r = beg + threadIdx.x; r < end; r += blockDim.x) {
-            K k;
-            uint32_t v;
-            load_kv(b, sg.src & 3u, r, k, v);
-            b.k0[r] = k;
-            b.v0[r] = v;
-        }
+        for (uint64_t r = beg + threadIdx.x; r < end; r += blockDim.x) copy_row(b, sg, r);
     }
 }
 
@@ -1074,6 +1111,8 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
     Bufs<K> b;
     b.ext_bank = (const K *)a.bank;
     b.ext_order = a.order_in;
+    b.flags = a.flags;
+    b.write_keys = a.flags == nullptr;
     void *p = nullptr;
     int rc;
     if (a.keys_out) {
@@ -1132,6 +1171,7 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
         lists.copy = cc.take<LargeSeg>(cap_copy);
         lists.copy_large = cc.take<LargeSeg>(cap_large);
         lists.local_max = local_max;
+        lists.flags = a.flags;
     }
     // (a segment's chunks <= its rows / chunk_rows + 1)
     LevelRefs lr{};
@@ -1185,7 +1225,7 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
         { LaunchScope ls_(ctx, "classify");
             launch_k(classify_kernel<K>, grid, 256, 0, st, b, seg_start, d_nseg, n, a.key_bits, ctr, large[0], lists,
                      lr.top_hist, a.d_key_bits, a.d_in_order,
-                     a.keys_scratch && a.order_in == a.order_out);
+                     a.skip_single && a.order_in == a.order_out, a.flags && a.mark_starts);
         }
         FMCS_LAUNCH_CHECK("classify");
     }
@@ -1283,7 +1323,8 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
             }
         }
     }
-    // local tiers
+    // local tiers (they write flags or keys)
+    const bool fo = a.flags != nullptr;
     const size_t smem_a = kWarpsA * sizeof(OnchipSmem<K, 32, kItA>);
     const size_t smem_a2 = kWarpsA * sizeof(OnchipSmem<K, 32, kItA2>);
     const size_t smem_b1 = sizeof(OnchipSmem<K, kNtB1, kItB1>);
@@ -1292,14 +1333,17 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
     const size_t smem_c1b = sizeof(OnchipSmem<K, kNtC1b, kItC1b>);
     const size_t smem_c2 = sizeof(OnchipSmem<K, kNtC2, kItC2>);
     const size_t smem_c3 = sizeof(OnchipSmem<K, kNtC3, kItC3>);
-    if ((rc = set_smem(ctx, warp_sort_kernel<K, kItA>, smem_a))) return rc;
-    if ((rc = set_smem(ctx, warp_sort_kernel<K, kItA2>, smem_a2))) return rc;
-    if ((rc = set_smem(ctx, block_sort_kernel<K, kNtB1, kItB1>, smem_b1))) return rc;
-    if ((rc = set_smem(ctx, block_sort_kernel<K, kNtB2, kItB2>, smem_b2))) return rc;
-    if ((rc = set_smem(ctx, block_sort_kernel<K, kNtC1, kItC1>, smem_c1))) return rc;
-    if ((rc = set_smem(ctx, block_sort_kernel<K, kNtC1b, kItC1b>, smem_c1b))) return rc;
-    if ((rc = set_smem(ctx, block_sort_kernel<K, kNtC2, kItC2>, smem_c2))) return rc;
-    if ((rc = set_smem(ctx, block_sort_kernel<K, kNtC3, kItC3>, smem_c3))) return rc;
+    auto set_smem2 = [&](auto *k0, auto *k1, size_t bytes) -> int {
+        return set_smem(ctx, fo ? k1 : k0, bytes);
+    };
+    if ((rc = set_smem2(warp_sort_kernel<K, kItA, false>, warp_sort_kernel<K, kItA, true>, smem_a))) return rc;
+    if ((rc = set_smem2(warp_sort_kernel<K, kItA2, false>, warp_sort_kernel<K, kItA2, true>, smem_a2))) return rc;
+    if ((rc = set_smem2(block_sort_kernel<K, kNtB1, kItB1, false>, block_sort_kernel<K, kNtB1, kItB1, true>, smem_b1))) return rc;
+    if ((rc = set_smem2(block_sort_kernel<K, kNtB2, kItB2, false>, block_sort_kernel<K, kNtB2, kItB2, true>, smem_b2))) return rc;
+    if ((rc = set_smem2(block_sort_kernel<K, kNtC1, kItC1, false>, block_sort_kernel<K, kNtC1, kItC1, true>, smem_c1))) return rc;
+    if ((rc = set_smem2(block_sort_kernel<K, kNtC1b, kItC1b, false>, block_sort_kernel<K, kNtC1b, kItC1b, true>, smem_c1b))) return rc;
+    if ((rc = set_smem2(block_sort_kernel<K, kNtC2, kItC2, false>, block_sort_kernel<K, kNtC2, kItC2, true>, smem_c2))) return rc;
+    if ((rc = set_smem2(block_sort_kernel<K, kNtC3, kItC3, false>, block_sort_kernel<K, kNtC3, kItC3, true>, smem_c3))) return rc;
     // Each tier's launch, with the counter word of its list.  An eager call
     // that knows the lists' sizes from its last read-back (tiers_known) does
     // not launch a tier whose list is empty.  A captured graph launches every
@@ -1312,50 +1356,50 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
     std::vector<Tier> tiers;
     tiers.push_back({kCtrLocalT, [&](cudaStream_t s, bool early) {
         LaunchScope ls_(ctx, "thread_sort");
-        launch_on(early, thread_sort_kernel<K, 16>, sms * 8, 256, 0, s, b, lists.t, &ctr[kCtrLocalT]);
+        launch_on(early, fo ? thread_sort_kernel<K, 16, true> : thread_sort_kernel<K, 16, false>, sms * 8, 256, 0, s, b, lists.t, &ctr[kCtrLocalT]);
     }});
     if constexpr (sizeof(K) <= 4) {
         tiers.push_back({kCtrLocalT32, [&](cudaStream_t s, bool early) {
             LaunchScope ls_(ctx, "thread_sort_32");
-            launch_on(early, thread_sort_kernel<K, 32>, sms * 8, 256, 0, s, b, lists.t32, &ctr[kCtrLocalT32]);
+            launch_on(early, fo ? thread_sort_kernel<K, 32, true> : thread_sort_kernel<K, 32, false>, sms * 8, 256, 0, s, b, lists.t32, &ctr[kCtrLocalT32]);
         }});
     }
     tiers.push_back({kCtrLocalA, [&](cudaStream_t s, bool early) {
         LaunchScope ls_(ctx, "warp_sort");
-        launch_on(early, warp_sort_kernel<K, kItA>, sms * warp_ctas_per_sm(kItA), kWarpsA * 32, smem_a, s, b, lists.a, &ctr[kCtrLocalA]);
+        launch_on(early, fo ? warp_sort_kernel<K, kItA, true> : warp_sort_kernel<K, kItA, false>, sms * warp_ctas_per_sm(kItA), kWarpsA * 32, smem_a, s, b, lists.a, &ctr[kCtrLocalA]);
     }});
     tiers.push_back({kCtrLocalA2, [&](cudaStream_t s, bool early) {
         LaunchScope ls_(ctx, "warp_sort_256");
-        launch_on(early, warp_sort_kernel<K, kItA2>, sms * warp_ctas_per_sm(kItA2), kWarpsA * 32, smem_a2, s, b, lists.a2, &ctr[kCtrLocalA2]);
+        launch_on(early, fo ? warp_sort_kernel<K, kItA2, true> : warp_sort_kernel<K, kItA2, false>, sms * warp_ctas_per_sm(kItA2), kWarpsA * 32, smem_a2, s, b, lists.a2, &ctr[kCtrLocalA2]);
     }});
     tiers.push_back({kCtrLocalB1, [&](cudaStream_t s, bool early) {
         LaunchScope ls_(ctx, "block_sort_512");
-        launch_on(early, block_sort_kernel<K, kNtB1, kItB1>, sms * (1024 / kNtB1), kNtB1, smem_b1, s, b, lists.b1,
+        launch_on(early, fo ? block_sort_kernel<K, kNtB1, kItB1, true> : block_sort_kernel<K, kNtB1, kItB1, false>, sms * (1024 / kNtB1), kNtB1, smem_b1, s, b, lists.b1,
                   &ctr[kCtrLocalB1]);
     }});
     tiers.push_back({kCtrLocalB2, [&](cudaStream_t s, bool early) {
         LaunchScope ls_(ctx, "block_sort_1024");
-        launch_on(early, block_sort_kernel<K, kNtB2, kItB2>, sms * (1024 / kNtB2), kNtB2, smem_b2, s, b, lists.b2,
+        launch_on(early, fo ? block_sort_kernel<K, kNtB2, kItB2, true> : block_sort_kernel<K, kNtB2, kItB2, false>, sms * (1024 / kNtB2), kNtB2, smem_b2, s, b, lists.b2,
                  &ctr[kCtrLocalB2]);
     }});
     tiers.push_back({kCtrLocalC1, [&](cudaStream_t s, bool early) {
         LaunchScope ls_(ctx, "block_sort_2048");
-        launch_on(early, block_sort_kernel<K, kNtC1, kItC1>, sms * (1024 / kNtC1), kNtC1, smem_c1, s, b, lists.c1,
+        launch_on(early, fo ? block_sort_kernel<K, kNtC1, kItC1, true> : block_sort_kernel<K, kNtC1, kItC1, false>, sms * (1024 / kNtC1), kNtC1, smem_c1, s, b, lists.c1,
                  &ctr[kCtrLocalC1]);
     }});
     tiers.push_back({kCtrLocalC1b, [&](cudaStream_t s, bool early) {
         LaunchScope ls_(ctx, "block_sort_2304");
-        launch_on(early, block_sort_kernel<K, kNtC1b, kItC1b>, sms * (1024 / kNtC1b), kNtC1b, smem_c1b, s, b, lists.c1b,
+        launch_on(early, fo ? block_sort_kernel<K, kNtC1b, kItC1b, true> : block_sort_kernel<K, kNtC1b, kItC1b, false>, sms * (1024 / kNtC1b), kNtC1b, smem_c1b, s, b, lists.c1b,
                  &ctr[kCtrLocalC1b]);
     }});
     tiers.push_back({kCtrLocalC2, [&](cudaStream_t s, bool early) {
         LaunchScope ls_(ctx, "block_sort_4096");
-        launch_on(early, block_sort_kernel<K, kNtC2, kItC2>, sms * (1024 / kNtC2), kNtC2, smem_c2, s, b, lists.c2,
+        launch_on(early, fo ? block_sort_kernel<K, kNtC2, kItC2, true> : block_sort_kernel<K, kNtC2, kItC2, false>, sms * (1024 / kNtC2), kNtC2, smem_c2, s, b, lists.c2,
                  &ctr[kCtrLocalC2]);
     }});
     tiers.push_back({kCtrLocalC3, [&](cudaStream_t s, bool early) {
         LaunchScope ls_(ctx, "block_sort_8192");
-        launch_on(early, block_sort_kernel<K, kNtC3, kItC3>, sms * (1024 / kNtC3), kNtC3, smem_c3, s, b, lists.c3,
+        launch_on(early, fo ? block_sort_kernel<K, kNtC3, kItC3, true> : block_sort_kernel<K, kNtC3, kItC3, false>, sms * (1024 / kNtC3), kNtC3, smem_c3, s, b, lists.c3,
                  &ctr[kCtrLocalC3]);
     }});
     tiers.push_back({kCtrCopy, [&](cudaStream_t s, bool early) {
@@ -1454,6 +1498,8 @@ int lsd_sort_full_t(fmcs_ctx *ctx, void *keys, uint32_t *vals, uint64_t n, uint3
     b.v0 = vals;
     b.ext_bank = nullptr;
     b.ext_order = nullptr;
+    b.flags = nullptr;
+    b.write_keys = 1;
     if ((rc = ws_get(ctx, kSlotKeys1, n * sizeof(K), &p))) return rc;
     b.k1 = (K *)p;
     if ((rc = ws_get(ctx, kSlotVals1, n * sizeof(uint32_t), &p))) return rc;
