@@ -518,39 +518,40 @@ __global__ void __launch_bounds__(kNtM, kHistCtas) msd_hist_kernel(Bufs<K> b, Le
     LargeSeg sg = segs[s];
     uint32_t sfirst = r.chunk_prefix[s], snext = r.chunk_prefix[s + 1];
     uint32_t prow = 0, psup = 0;   // the chunk to write out
-    // up to MAXJ rows a thread of [beg, end) of the segment; the source switch
-    // is taken once a tile
-    auto load_tile = [&](K (&key)[MAXJ], uint32_t beg, uint32_t end) {
+    // up to MAXJ rows a thread of the `rows` rows of the segment from row `beg`;
+    // the source switch is taken once a tile
+    auto load_tile = [&](K (&key)[MAXJ], uint32_t beg, uint32_t rows) {
+        const uint64_t at = (uint64_t)sg.start + beg;
         if (sg.src == kSrcExt && b.ext_order) {
-            const uint32_t *os = b.ext_order + sg.start;
+            const uint32_t *os = b.ext_order + at;
             uint32_t v[MAXJ];
 #pragma unroll
             for (int j = 0; j < MAXJ; ++j) {
-                const uint32_t i = beg + threadIdx.x + j * kNtM;
-                v[j] = i < end ? os[i] : 0u;
+                const uint32_t i = threadIdx.x + j * kNtM;
+                v[j] = i < rows ? os[i] : 0u;
             }
 #pragma unroll
             for (int j = 0; j < MAXJ; ++j) {
-                const uint32_t i = beg + threadIdx.x + j * kNtM;
-                key[j] = i < end ? b.ext_bank[v[j]] : K(0);
+                const uint32_t i = threadIdx.x + j * kNtM;
+                key[j] = i < rows ? b.ext_bank[v[j]] : K(0);
             }
             if (r.gathered) {
                 // the scatter reads them in order instead of gathering again
                 // (32 bytes fetched a row): 60M rows in 64 groups, two rounds,
                 // 3.23 -> 2.54 ms
-                K *kd = b.k0 + sg.start;
+                K *kd = b.k0 + at;
 #pragma unroll
                 for (int j = 0; j < MAXJ; ++j) {
-                    const uint32_t i = beg + threadIdx.x + j * kNtM;
-                    if (i < end) kd[i] = key[j];
+                    const uint32_t i = threadIdx.x + j * kNtM;
+                    if (i < rows) kd[i] = key[j];
                 }
             }
         } else {
-            const K *ks = (sg.src == kSrcExt ? b.ext_bank : sg.src == kSrcBuf1 ? b.k1 : b.k0) + sg.start;
+            const K *ks = (sg.src == kSrcExt ? b.ext_bank : sg.src == kSrcBuf1 ? b.k1 : b.k0) + at;
 #pragma unroll
             for (int j = 0; j < MAXJ; ++j) {
-                const uint32_t i = beg + threadIdx.x + j * kNtM;
-                key[j] = i < end ? ks[i] : K(0);
+                const uint32_t i = threadIdx.x + j * kNtM;
+                key[j] = i < rows ? ks[i] : K(0);
             }
         }
     };
@@ -558,7 +559,7 @@ __global__ void __launch_bounds__(kNtM, kHistCtas) msd_hist_kernel(Bufs<K> b, Le
     for (uint32_t q = q0; q <= q1; ++q) {
         const uint32_t set = (q - q0) & 1u;
         K key[MAXJ];
-        uint32_t beg = 0, end = 0, lo = 0, width = 0;
+        uint32_t beg = 0, rows = 0, lo = 0, width = 0;   // (rows left: a row's index may end at 2^32 - 1)
         if (q < q1) {
             if (q >= snext) {   // every large segment has a chunk: the next chunk starts the next segment
                 ++s;
@@ -568,10 +569,9 @@ __global__ void __launch_bounds__(kNtM, kHistCtas) msd_hist_kernel(Bufs<K> b, Le
             }
             width = sg.shift < (uint32_t)kRadixBits ? sg.shift : (uint32_t)kRadixBits;
             lo = sg.shift - width;
-            const uint32_t o = (q - sfirst) * r.chunk_rows;
-            beg = o;
-            end = o + min(r.chunk_rows, sg.len - o);
-            load_tile(key, beg, end);
+            beg = (q - sfirst) * r.chunk_rows;
+            rows = min(r.chunk_rows, sg.len - beg);
+            load_tile(key, beg, rows);
         }
         if (q > q0) {
             // the chunk before, counted in the other set
@@ -589,12 +589,13 @@ __global__ void __launch_bounds__(kNtM, kHistCtas) msd_hist_kernel(Bufs<K> b, Le
         for (;;) {
 #pragma unroll
             for (int j = 0; j < MAXJ; ++j) {
-                const uint32_t i = beg + threadIdx.x + j * kNtM;
-                if (i < end) atomicAdd(&sh[set][warp][digit_of(key[j], lo, width)], 1u);
+                const uint32_t i = threadIdx.x + j * kNtM;
+                if (i < rows) atomicAdd(&sh[set][warp][digit_of(key[j], lo, width)], 1u);
             }
+            if (rows <= MAXJ * kNtM) break;
+            rows -= MAXJ * kNtM;
             beg += MAXJ * kNtM;
-            if (beg >= end) break;
-            load_tile(key, beg, end);
+            load_tile(key, beg, rows);
         }
         prow = q;
         psup = super_row(sfirst, s) + (q - sfirst) / kSuper;
