@@ -685,11 +685,11 @@ __global__ void instance_bases_kernel(const uint32_t *starts, uint32_t ninst, co
 __global__ void __launch_bounds__(256) localize_kernel(const uint32_t *__restrict__ starts, uint32_t ninst,
                                                        const uint32_t *__restrict__ base_of,
                                                        uint32_t *__restrict__ order, uint32_t *__restrict__ group,
-                                                       uint64_t n, bool vec)
+                                                       uint64_t n, uint32_t rows, bool vec)
 {
     kernel_prologue();
-    for (uint64_t base = blockIdx.x * (uint64_t)kInstRows; base < n; base += (uint64_t)gridDim.x * kInstRows) {
-        const uint64_t end = min(n, base + kInstRows);
+    for (uint64_t base = blockIdx.x * (uint64_t)rows; base < n; base += (uint64_t)gridDim.x * rows) {
+        const uint64_t end = min(n, base + rows);
         const uint32_t lo = find_segment_warp(starts, ninst, (uint32_t)base);
         const uint32_t hi = find_segment_warp(starts, ninst, (uint32_t)(end - 1));
         for (uint64_t i = base + threadIdx.x * 4; i < end; i += blockDim.x * 4) {
@@ -867,9 +867,12 @@ extern "C" int fmcs_run_batch(fmcs_ctx *ctx, const void *const *cols, const uint
     }
     {
         LaunchScope ls_(ctx, "localize");
-        launch_k(localize_kernel, ctx->num_sms * 8, 256, 0, st, (const uint32_t *)d_starts, ninst,
-                 (const uint32_t *)d_base, (uint32_t *)dorder, group, n,
-                 (((uintptr_t)dorder | (uintptr_t)group) & 15u) == 0);
+        // short runs of rows where long ones would leave SMs idle
+        const uint32_t rows = n < (uint64_t)ctx->num_sms * 8 * kInstRows ? 1024u : kInstRows;
+        const uint64_t tiles = (n + rows - 1) / rows;
+        launch_k(localize_kernel, (unsigned)std::min<uint64_t>(tiles, ctx->num_sms * 8), 256, 0, st,
+                 (const uint32_t *)d_starts, ninst, (const uint32_t *)d_base, (uint32_t *)dorder, group, n,
+                 rows, (((uintptr_t)dorder | (uintptr_t)group) & 15u) == 0);
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "fmcs_run_batch localize");
