@@ -29,6 +29,7 @@
 #include "device_common.cuh"
 #include "fmcs_internal.h"
 #include "onchip.cuh"
+#include "sort_lists.h"
 
 #include <algorithm>
 #include <functional>
@@ -75,7 +76,6 @@ constexpr int kCtrLocalT = 11;
 constexpr int kCtrLocalT32 = 14;
 constexpr int kCtrCopyLarge = 12;   // copy entries larger than kCopySplit rows
 constexpr int kCtrCopyTile = 13;
-constexpr uint32_t kCopySplit = 4096;
 constexpr int kCtrLevel = 15;      // MSD levels started so far (device-side level index)
 constexpr int kCtrLocalC3 = 16;
 constexpr int kCtrLocalC1b = 17;
@@ -1130,16 +1130,13 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
 
     // lists (capacities are bounds on disjoint segments of each tier's minimum size)
     const uint32_t local_max = std::max<uint32_t>(kCapA, std::min<uint32_t>(ctx->local_max, kCapLocal));
-    const uint64_t cap_large = n / (local_max + 1) + 2;
+    const SortListCaps caps = sort_list_caps(n, local_max, a.key_bits);
+    const uint64_t cap_large = caps.large;
     const uint64_t cap_t = n / 2 + 2, cap_t32 = n / (kCapT + 1) + 2, cap_a = n / (kCapT + 1) + 2;
     const uint64_t cap_a2 = n / (kCapA + 1) + 2, cap_b1 = n / (kCapA2 + 1) + 2;
     const uint64_t cap_b2 = n / (kCapB1 + 1) + 2;
     const uint64_t cap_c1 = n / (kCapB2 + 1) + 2, cap_c1b = n / (kCapC1 + 1) + 2, cap_c2 = n / (kCapC1b + 1) + 2;
     const uint64_t cap_c3 = n / (kCapC2 + 1) + 2;
-    // copy entries: disjoint ranges; at most 256 children per large segment per
-    // level, so bounded by both n and (levels + 1) * 256 * cap_large
-    const uint64_t levels_max = (a.key_bits + kRadixBits - 1) / kRadixBits;
-    const uint64_t cap_copy = std::min<uint64_t>(n, (levels_max + 1) * kRadix * cap_large) + 2;
     LargeSeg *large[2];
     if ((rc = ws_get(ctx, kSlotLarge0, cap_large * sizeof(LargeSeg), &p))) return rc;
     large[0] = (LargeSeg *)p;
@@ -1165,12 +1162,12 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
         lists.c1b = cv.take<uint2>(cap_c1b);
         lists.c2 = cv.take<uint2>(cap_c2);
         lists.c3 = cv.take<uint2>(cap_c3);
-        if ((rc = ws_get(ctx, kSlotLocalC, carve_total({cap_copy * sizeof(LargeSeg), cap_large * sizeof(LargeSeg)}),
+        if ((rc = ws_get(ctx, kSlotLocalC, carve_total({caps.copy * sizeof(LargeSeg), caps.copy_large * sizeof(LargeSeg)}),
                          &p)))
             return rc;
         Carver cc(p);
-        lists.copy = cc.take<LargeSeg>(cap_copy);
-        lists.copy_large = cc.take<LargeSeg>(cap_large);
+        lists.copy = cc.take<LargeSeg>(caps.copy);
+        lists.copy_large = cc.take<LargeSeg>(caps.copy_large);
         lists.local_max = local_max;
         lists.flags = a.flags;
     }
@@ -1197,13 +1194,13 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
         lr.work = cv.take<Chunk>(cap_chunks);
         lr.long_rows = cv.take<uint2>(cap_long);
     }
-    uint32_t *tile_prefix;
-    if ((rc = ws_get(ctx, kSlotTilePrefix, carve_total({(cap_large + 1) * sizeof(uint32_t),
+    uint32_t *tile_prefix;   // of the large copies
+    if ((rc = ws_get(ctx, kSlotTilePrefix, carve_total({(caps.copy_large + 1) * sizeof(uint32_t),
                                                         (cap_large + 1) * sizeof(uint32_t)}), &p)))
         return rc;
     {
         Carver cv(p);
-        tile_prefix = cv.take<uint32_t>(cap_large + 1);
+        tile_prefix = cv.take<uint32_t>(caps.copy_large + 1);
         lr.chunk_prefix = cv.take<uint32_t>(cap_large + 1);
     }
     uint32_t *ctr;
