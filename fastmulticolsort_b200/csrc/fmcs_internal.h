@@ -247,7 +247,7 @@ struct SortArgs {
     // Device-side overrides read by the round's first kernel (no host
     // read-back): the significant key bits (<= key_bits, which then only
     // bounds the number of radix levels), and a flag that, when non-zero,
-    // says the rows are in order already (every segment is only copied).
+    // says the rows are in order already (they are only copied; not with flags).
     const uint32_t *d_key_bits = nullptr;
     const uint32_t *d_in_order = nullptr;
     // flags (n bytes, or NULL): 1 where a group of equal keys starts inside its

@@ -327,7 +327,20 @@ __global__ void classify_kernel(Bufs<K> b, const uint32_t *__restrict__ seg_star
 {
     kernel_prologue();
     if (d_key_bits) key_bits = min(key_bits, *d_key_bits);
-    if (d_in_order && *d_in_order) key_bits = 0;   // every segment is in order: copy only
+    if (d_in_order && *d_in_order) {
+        // Every segment is in order: the rows keep their places, and their keys and
+        // oids go to BUF0 here.  (No segment is listed: there may be one per two
+        // rows, many more than the levels' finished segments, which the copy lists
+        // are sized for.)
+        for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+            K k;
+            uint32_t v;
+            load_kv(b, kSrcExt, i, k, v);
+            b.k0[i] = k;
+            b.v0[i] = v;
+        }
+        return;
+    }
     if (!seg_start && top_hist && n > lists.local_max) {
         // round 0 over the whole array with its first-level histogram already
         // counted (level 0's msd_plan reads the stitch's rows): the one large
@@ -1220,6 +1233,7 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
         unsigned grid = seg_start ? (unsigned)std::min<uint64_t>((a.nseg_host + 255) / 256 + 1, (uint64_t)sms * 16)
                                   : 1u;
         if (seg_start && a.nseg_host == 0) grid = (unsigned)sms * 16;
+        if (a.d_in_order) grid = std::max(grid, (unsigned)sms * 4);   // (it may copy every row)
         { LaunchScope ls_(ctx, "classify");
             launch_k(classify_kernel<K>, grid, 256, 0, st, b, seg_start, d_nseg, n, a.key_bits, ctr, large[0], lists,
                      lr.top_hist, a.d_key_bits, a.d_in_order,
@@ -1608,6 +1622,7 @@ static int sort_dispatch(fmcs_ctx *ctx, const SortArgs &a)
 int sort_segments(fmcs_ctx *ctx, const SortArgs &a)
 {
     if (a.n == 0) return FMCS_OK;
+    if (a.flags && a.d_in_order) return set_error(ctx, FMCS_E_INVAL, "sort: rows that may be in order have no flags");
     if (a.key_bits == 0 || a.key_bits > 8 * a.bank_bytes)
         return set_error(ctx, FMCS_E_INVAL, "sort: key_bits must be in 1..8*bank_bytes");
     switch (a.bank_bytes) {
