@@ -26,11 +26,14 @@ namespace {
 // refined: the rows of each bucket of 16 or more are spread over as many places
 // by the 32 bits after the digit, interpolated between the lowest and highest
 // that a sample of the bucket shows.  When some bucket even then holds more
-// than kBucketMax rows, step 1 is done again: NT splitters, compounds taken at even positions
-// and sorted across the group by a bitonic network, cut the rows into coarse
-// buckets of about IT rows whatever the keys (binary search), and a coarse
-// bucket of m rows is cut into m fine ones by interpolating between its two
-// splitters.  Every step keeps the compounds' order.
+// than kBucketMax rows, step 1 is done again: NT splitters, one compound taken
+// somewhere in each NT-th of the segment and sorted across the group by a bitonic
+// network, cut the rows into coarse buckets of about IT rows whatever the keys
+// (binary search), and a coarse bucket of m rows is cut into m fine ones by
+// interpolating between its two splitters.  Every step keeps the compounds' order.
+// Should some bucket hold more than kBucketWorst rows after all (keys laid out
+// against the sampled places), the whole segment is sorted by a network instead:
+// step 3 is quadratic in a bucket's rows.
 // The oids wait in shared memory in the order they were read; a compound's
 // position bits find a row's oid when the segment is written out, so only
 // compounds move.
@@ -52,6 +55,9 @@ constexpr uint32_t kBucketMax = 64;
 // kBucketRefine: 24 (16 and 40 differ by 1 to 2%, either way by case; without the
 // step the 90,001 rows take 198 us instead of 175).
 constexpr uint32_t kBucketRefine = 24;
+// kBucketWorst: coarse buckets hold IT rows on average, at random places hardly
+// ever ten times as many.
+constexpr uint32_t kBucketWorst = 128;
 
 constexpr int pow2_ceil(int x)
 {
@@ -269,6 +275,22 @@ __device__ __forceinline__ bool comp_less(const OnchipSmem<K, NT, IT> &sm, unsig
     return less;
 }
 
+// Where splitter t of len rows is taken: somewhere in the t-th of NT equal parts.
+// (The parts' beginnings are an even stride apart.  Rows whose keys repeat with a
+// period that shares a factor with it, as in joined or generated tables, would
+// show a few of their keys only, and the rows of all others would share a bucket:
+// a round over 296 segments of 8192 rows, codes i % 8 and one far key each, 3.35
+// ms with places at the beginnings and 0.18 with these; 64-bit keys of a few low
+// bits and one highest 18.8 and 0.32.)
+template <int NT>
+__device__ __forceinline__ uint32_t splitter_place(uint32_t t, uint32_t len)
+{
+    const uint32_t a = t * len / NT, z = (t + 1) * len / NT;   // (len <= 2^13)
+    uint32_t h = (t + 1) * 0x9E3779B9u;   // mixed: an odd constant, a fold, another
+    h = (h ^ (h >> 15)) * 0x2C1B3C6Du;
+    return a + __umulhi(h, z - a);
+}
+
 // The splitters of step 1's second try: NT compounds of the segment (in sm.cs
 // by position), sorted into sm.spl.  Out of line: it runs for skewed segments
 // only, and its registers must not weigh on the others.
@@ -276,7 +298,7 @@ template <typename K, int NT, int IT>
 __device__ __noinline__ void sort_splitters(OnchipSmem<K, NT, IT> &sm, uint32_t len, uint32_t drop, uint32_t nbits)
 {
     const uint32_t tid = NT == 32 ? lane_id() : threadIdx.x;
-    unsigned long long x = sm.cs[(uint32_t)(((uint64_t)tid * len) / NT)];
+    unsigned long long x = sm.cs[splitter_place<NT>(tid, len)];
 #pragma unroll 1
     for (uint32_t k = 2; k <= (uint32_t)NT; k <<= 1) {
 #pragma unroll 1
@@ -295,6 +317,37 @@ __device__ __noinline__ void sort_splitters(OnchipSmem<K, NT, IT> &sm, uint32_t 
         }
     }
     sm.spl[tid] = x;
+}
+
+// The compounds in sm.cs sorted in place, len of them, 2^nbits >= len: a bitonic
+// network whose comparisons all point upwards (each merge starts by comparing
+// mirrored places), so that the places past len need not exist.  91 steps for
+// 8192 rows whatever the keys; it runs for keys that defeat the splitters only.
+template <typename K, int NT, int IT>
+__device__ __noinline__ void sort_network(OnchipSmem<K, NT, IT> &sm, uint32_t len, uint32_t drop, uint32_t nbits)
+{
+    const uint32_t tid = NT == 32 ? lane_id() : threadIdx.x;
+    const uint32_t half = 1u << (nbits - 1u);
+#pragma unroll 1
+    for (uint32_t k = 2; k <= 2u * half; k <<= 1) {
+#pragma unroll 1
+        for (uint32_t h = k >> 1; h > 0; h >>= 1) {
+            group_sync<NT>();
+#pragma unroll 1
+            for (uint32_t t = tid; t < half; t += NT) {
+                const uint32_t i = 2u * t - (t & (h - 1u));   // bit h of the place is 0
+                const uint32_t j = h == k >> 1 ? i ^ (k - 1u) : i + h;
+                if (j < len) {
+                    const unsigned long long x = sm.cs[i], y = sm.cs[j];
+                    if (comp_less(sm, y, x, drop, nbits)) {
+                        sm.cs[i] = y;
+                        sm.cs[j] = x;
+                    }
+                }
+            }
+        }
+    }
+    group_sync<NT>();
 }
 
 // The compounds' layout, for reading sm.cs back.
@@ -492,7 +545,10 @@ __device__ __forceinline__ OnchipInfo onchip_core(OnchipSmem<K, NT, IT> &sm, uns
                 bk[j] = (fb << 16) | atomicAdd(&sm.off[fb], 1u);
             }
         }
-        group_scan_bins<K, NT, IT>(sm, nb, len);
+        if (group_scan_bins<K, NT, IT>(sm, nb, len) > kBucketWorst) {   // (uniform across the group)
+            sort_network<K, NT, IT>(sm, len, drop, nbits);
+            return OnchipInfo{prefix, nbits, drop, false};
+        }
     }
     // rows land bucketed; each keeps its bucket's start and size
 #pragma unroll
