@@ -231,6 +231,7 @@ int plan_pipeline(fmcs_ctx *ctx, const Plan &plan, const void *const *dcols, con
         return launch_stitch(ctx, sl.data(), (int)sl.size(), *bank_out, bp.bytes, n, th, bp.bits, chunk_rows, s);
     };
     void *next_bank = nullptr;   // the next round's bank, stitched on the second stream
+    ParFork side(ctx, ctx->stream);
     for (uint32_t b = 0; b < nbanks; ++b) {
         const BankPlan &bp = plan.banks[b];
         const bool last = (b + 1 == nbanks);
@@ -239,12 +240,12 @@ int plan_pipeline(fmcs_ctx *ctx, const Plan &plan, const void *const *dcols, con
         if (next_bank) {
             bank = next_bank;
             next_bank = nullptr;
-            if ((rc = join_par(ctx, ctx->stream))) return rc;
+            if ((rc = side.join())) return rc;
         } else if ((rc = stitch_bank(b, nullptr, &bank))) {
             return rc;
         }
         if (!last && !ctx->prof_on) {
-            if ((rc = fork_par(ctx, ctx->stream))) return rc;
+            if ((rc = side.fork())) return rc;
             if ((rc = stitch_bank(b + 1, ctx->par, &next_bank))) return rc;
         }
         if (b > 0) top_hist = nullptr;
@@ -836,6 +837,7 @@ extern "C" int fmcs_run_batch(fmcs_ctx *ctx, const void *const *cols, const uint
         return launch_stitch(ctx, sl.data(), (int)sl.size(), *bank_out, bp.bytes, n, nullptr, 0, 0, s);
     };
     void *next_bank = nullptr;
+    ParFork side(ctx, ctx->stream);
     for (uint32_t b = 0; b < nbanks; ++b) {
         const BankPlan &bp = plan.banks[b];
         const bool last = (b + 1 == nbanks);
@@ -844,12 +846,12 @@ extern "C" int fmcs_run_batch(fmcs_ctx *ctx, const void *const *cols, const uint
         if (next_bank) {
             bank = next_bank;
             next_bank = nullptr;
-            if ((rc = join_par(ctx, ctx->stream))) return rc;
+            if ((rc = side.join())) return rc;
         } else if ((rc = stitch_bank(b, nullptr, &bank))) {
             return rc;
         }
         if (!last && !ctx->prof_on) {
-            if ((rc = fork_par(ctx, ctx->stream))) return rc;
+            if ((rc = side.fork())) return rc;
             if ((rc = stitch_bank(b + 1, ctx->par, &next_bank))) return rc;
         }
         uint32_t *ns = last ? nullptr : segs[b & 1];

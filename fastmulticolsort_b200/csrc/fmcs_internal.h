@@ -172,6 +172,31 @@ int capture_while(fmcs_ctx *ctx, cudaStream_t st,
 int par_stream(fmcs_ctx *ctx, cudaStream_t *par);
 int fork_par(fmcs_ctx *ctx, cudaStream_t st);
 int join_par(fmcs_ctx *ctx, cudaStream_t st);
+// A fork that outlives the statements around it: joined on every way out, so
+// that after a call that failed half-way the work on `par` (it reads the caller's
+// columns and writes the workspace) still comes before the context's next call.
+class ParFork {
+  public:
+    ParFork(fmcs_ctx *ctx, cudaStream_t st) : ctx_(ctx), st_(st) {}
+    ~ParFork() { join(); }
+    int fork()
+    {
+        const int rc = fork_par(ctx_, st_);
+        open_ = rc == 0;
+        return rc;
+    }
+    int join()
+    {
+        const bool open = open_;
+        open_ = false;
+        return open ? join_par(ctx_, st_) : 0;
+    }
+
+  private:
+    fmcs_ctx *ctx_;
+    cudaStream_t st_;
+    bool open_ = false;
+};
 
 // Launches a library kernel with programmatic stream serialization: it may
 // begin launching while the stream's previous kernel finishes (its prologue
