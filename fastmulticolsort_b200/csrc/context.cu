@@ -29,6 +29,16 @@ int cuda_fail(fmcs_ctx *ctx, cudaError_t e, const char *what)
     return set_error(ctx, e == cudaErrorMemoryAllocation ? FMCS_E_OOM : FMCS_E_CUDA, buf);
 }
 
+int raise_smem(fmcs_ctx *ctx, const void *kernel, size_t bytes)
+{
+    for (const void *k : ctx->smem_raised)
+        if (k == kernel) return FMCS_OK;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel shared memory limit");
+    ctx->smem_raised.push_back(kernel);
+    return FMCS_OK;
+}
+
 int ws_get(fmcs_ctx *ctx, int slot, size_t bytes, void **out)
 {
     Workspace &w = ctx->ws;

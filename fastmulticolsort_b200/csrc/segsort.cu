@@ -1103,13 +1103,6 @@ __global__ void __launch_bounds__(256) copy_tiles_kernel(Bufs<K> b, const LargeS
     }
 }
 
-template <typename F>
-int set_smem(fmcs_ctx *ctx, F *f, size_t bytes)
-{
-    cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    return e == cudaSuccess ? FMCS_OK : cuda_fail(ctx, e, "cudaFuncSetAttribute");
-}
-
 #define FMCS_LAUNCH_CHECK(what)                                         \
     do {                                                                \
         cudaError_t e_ = cudaGetLastError();                            \
@@ -1274,7 +1267,7 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
     // MSD levels
     const int levels = (int)((a.key_bits + kRadixBits - 1) / kRadixBits);
     const size_t msd_smem = sizeof(MsdSmem<K, IT>);
-    if ((rc = set_smem(ctx, msd_scatter_kernel<K, RANK, IT>, msd_smem))) return rc;
+    if ((rc = raise_smem(ctx, (const void *)msd_scatter_kernel<K, RANK, IT>, msd_smem))) return rc;
     if (n > (uint64_t)local_max) {
         // Host-known count of the level's large segments (exact unless the
         // caller asked for a fixed launch sequence, e.g. for graph capture).
@@ -1346,7 +1339,7 @@ int sort_segments_t(fmcs_ctx *ctx, const SortArgs &a)
     const size_t smem_c2 = sizeof(OnchipSmem<K, kNtC2, kItC2>);
     const size_t smem_c3 = sizeof(OnchipSmem<K, kNtC3, kItC3>);
     auto set_smem2 = [&](auto *k0, auto *k1, size_t bytes) -> int {
-        return set_smem(ctx, fo ? k1 : k0, bytes);
+        return raise_smem(ctx, (const void *)(fo ? k1 : k0), bytes);
     };
     if ((rc = set_smem2(warp_sort_kernel<K, kItA, false>, warp_sort_kernel<K, kItA, true>, smem_a))) return rc;
     if ((rc = set_smem2(warp_sort_kernel<K, kItA2, false>, warp_sort_kernel<K, kItA2, true>, smem_a2))) return rc;
@@ -1556,7 +1549,7 @@ int lsd_sort_full_t(fmcs_ctx *ctx, void *keys, uint32_t *vals, uint64_t n, uint3
     ctr = (uint32_t *)p + 64;
     lr.ctr = ctr;
     const size_t msd_smem = sizeof(MsdSmem<K, IT>);
-    if ((rc = set_smem(ctx, msd_scatter_kernel<K, RANK, IT>, msd_smem))) return rc;
+    if ((rc = raise_smem(ctx, (const void *)msd_scatter_kernel<K, RANK, IT>, msd_smem))) return rc;
     const int sms = ctx->num_sms;
     Lists none{};
     int pass = 0;

@@ -217,24 +217,23 @@ __global__ void __launch_bounds__(NT, 1) small_plan_kernel(const __grid_constant
 }
 
 template <int NT, int IT>
-cudaError_t launch_small_t(fmcs_ctx *ctx, const SmallParams &p, const char *name)
+int launch_small_t(fmcs_ctx *ctx, const SmallParams &p, const char *name)
 {
     const size_t smem = sizeof(SmallSmem<NT, IT>);
-    cudaError_t e = cudaFuncSetAttribute(small_plan_kernel<NT, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
+    const int rc = raise_smem(ctx, (const void *)small_plan_kernel<NT, IT>, smem);
+    if (rc) return rc;
     LaunchScope ls_(ctx, name);
-    return launch_k(small_plan_kernel<NT, IT>, 1, NT, smem, ctx->stream, p);
+    const cudaError_t e = launch_k(small_plan_kernel<NT, IT>, 1, NT, smem, ctx->stream, p);
+    return e == cudaSuccess ? FMCS_OK : cuda_fail(ctx, e, "small plan launch");
 }
 
 int launch_small(fmcs_ctx *ctx, const SmallParams &p)
 {
     // as few rows a thread as the block allows: the steps are a serial chain
     // (profiled under the name of the on-chip tier of that capacity)
-    const cudaError_t e = p.n <= 1024   ? launch_small_t<256, 4>(ctx, p, "block_sort_1024")
-                          : p.n <= 4096 ? launch_small_t<1024, 4>(ctx, p, "block_sort_4096")
-                                        : launch_small_t<1024, 8>(ctx, p, "block_sort_8192");
-    return e == cudaSuccess ? FMCS_OK : cuda_fail(ctx, e, "small plan launch");
+    return p.n <= 1024   ? launch_small_t<256, 4>(ctx, p, "block_sort_1024")
+           : p.n <= 4096 ? launch_small_t<1024, 4>(ctx, p, "block_sort_4096")
+                         : launch_small_t<1024, 8>(ctx, p, "block_sort_8192");
 }
 
 }  // namespace

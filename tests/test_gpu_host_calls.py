@@ -1,0 +1,26 @@
+"""What a call asks of the CUDA runtime once its kernels and workspace are warm:
+nothing that locks other threads' launches out."""
+import numpy as np
+import pytest
+
+from fastmulticolsort_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,split", [(3_001, [50]), (60_000, [50]), (1_200_000, [17, 33])])
+def test_warm_calls_set_no_kernel_attributes(ctx, n, split):
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    cols, bw = W.cols_17b33(n, seed_index=5)
+    dev = [torch.from_numpy(c.view({4: np.int32, 8: np.int64}[c.itemsize])).cuda() for c in cols]
+    order, group = (torch.zeros(n, dtype=torch.int32, device="cuda") for _ in range(2))
+    for _ in range(2):
+        ctx.run_plan(dev, bw, split, order, group)
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+        ctx.run_plan(dev, bw, split, order, group)
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events()]
+    assert any("LaunchKernel" in x for x in names)   # runtime calls are recorded
+    assert not [x for x in names if "FuncSetAttribute" in x or x in ("cudaMalloc", "cudaFree")]
