@@ -13,6 +13,7 @@
 #include <fstream>
 #include <sstream>
 #include <cstring>
+#include <thread>
 
 namespace fmcs {
 
@@ -184,11 +185,19 @@ int launch_publish_counters(fmcs_ctx *ctx, const uint32_t *ctr, uint32_t seq)
     return e == cudaSuccess ? FMCS_OK : cuda_fail(ctx, e, "publish launch");
 }
 
+// The wait polls without a pause for a microsecond or two, then gives the core to
+// other threads between polls: on a host with fewer cores than server slots the
+// threads that submit and launch need it (30 Zipf requests at four slots: 6.03 ->
+// 4.14 ms on one core, 3.85 -> 2.89 on two, 2.62 -> 2.51 on four; the same on 16).
+constexpr uint32_t kSpinPolls = 1024;
+
 int wait_counters(fmcs_ctx *ctx, uint32_t seq, const char *what)
 {
     volatile const uint32_t *at = ctx->h_small + kHostSeq;
     for (uint32_t it = 1; *at != seq; ++it) {
-        if ((it & 1023u) != 0) continue;
+        if (it < kSpinPolls) continue;
+        std::this_thread::yield();
+        if ((it & 63u) != 0) continue;
         // now and then: has the stream failed, or ended without the counters?
         const cudaError_t e = cudaStreamQuery(ctx->stream);
         if (e == cudaErrorNotReady) continue;

@@ -24,3 +24,31 @@ def test_warm_calls_set_no_kernel_attributes(ctx, n, split):
     names = [e.name for e in prof.events()]
     assert any("LaunchKernel" in x for x in names)   # runtime calls are recorded
     assert not [x for x in names if "FuncSetAttribute" in x or x in ("cudaMalloc", "cudaFree")]
+
+
+def test_burst_on_one_host_core():
+    """Four server slots whose waits share one core with the submitting thread."""
+    import os
+    import torch
+    from fastmulticolsort_b200 import capi
+    from oracle import oracle as O
+    allowed = os.sched_getaffinity(0)
+    os.sched_setaffinity(0, {min(allowed)})   # threads started from here inherit it
+    try:
+        with capi.Server(0, slots=4, batch_rows_max=1 << 18) as server:
+            runs = []
+            for k in range(12):
+                cols, bw = W.cols_17b33(20_000 + 30_000 * k, seed_index=k)
+                dev = [torch.from_numpy(c.view({4: np.int32, 8: np.int64}[c.itemsize])).cuda() for c in cols]
+                order, group = (torch.zeros(cols[0].shape[0], dtype=torch.int32, device="cuda") for _ in range(2))
+                runs.append((cols, dev, order, group))
+            torch.cuda.synchronize()
+            tickets = [server.submit(dev, bw, order, group, split=[17, 33]) for _, dev, order, group in runs]
+            for t in tickets:
+                assert server.wait(t)["status"] == 0
+    finally:
+        os.sched_setaffinity(0, allowed)
+    for cols, _, order, group in runs:
+        o, g, _ = O.run_plan_sort(cols, bw, [17, 33])
+        assert np.array_equal(order.cpu().numpy().view(np.uint32), o)
+        assert np.array_equal(group.cpu().numpy().view(np.uint32), g)
