@@ -1526,7 +1526,12 @@ int lsd_sort_full_t(fmcs_ctx *ctx, void *keys, uint32_t *vals, uint64_t n, uint3
     LevelRefs lr{};
     lr.large[0] = seg;
     lr.large[1] = seg + 1;
-    lr.chunk_rows = msd_chunk_rows(ctx, n);
+    // (a pass's tiles have IT rows a thread whatever msd_items is.  As long as they
+    // all run at once a chunk is one tile: chunks of two make every CTA take them
+    // one after the other (300,000 rows of 50-bit keys: 284 us, one-tile chunks 217; 1.2M
+    // 311 and 270; 2M 330 and 343, 8M 861 and 889).)
+    const uint64_t tile = (uint64_t)kNtM * IT;
+    lr.chunk_rows = n <= tile * ctx->num_sms * msd_ctas_per_sm(IT) ? (uint32_t)tile : msd_chunk_rows(ctx, n);
     lr.max_chunks = (uint32_t)(n / lr.chunk_rows);
     const uint64_t chunks = (n - 1) / lr.chunk_rows + 1, supers = super_rows_max(chunks, 1);
     const size_t row = kRadix * sizeof(uint32_t);
