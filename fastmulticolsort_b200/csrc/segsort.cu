@@ -366,34 +366,38 @@ __global__ void classify_kernel(Bufs<K> b, const uint32_t *__restrict__ seg_star
         }
         return;
     }
-    // Four segments a thread, their starts in one 16-byte load (seg_start is
-    // 16-byte aligned): where most segments are one row (a round after nearly
-    // unique keys) this kernel only streams the starts.  67M of them: 126 us one
-    // segment a thread, 57 now.
+    // 128 segments a warp.  First four a lane, their starts in one 16-byte load
+    // (seg_start is 16-byte aligned): where all are one row and nobody reads their
+    // keys (a round after nearly unique keys) the kernel only streams the starts.
+    // 67M of them: 126 us one segment a thread, 57 so.  Otherwise the warp takes
+    // them 32 at a time, a lane each, so that neighbours stay neighbours in their
+    // list, as the tiers read it (four a lane made rounds of 2 to 16 rows a segment
+    // 4 to 8% slower).
     const uint32_t nseg = *d_nseg;
-    const uint32_t stride = gridDim.x * blockDim.x * 4;
-    for (uint64_t s0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4ull; s0 < nseg; s0 += stride) {
-        uint32_t at[5];
-        const uint32_t m = (uint32_t)min((uint64_t)4, nseg - s0);
-        if (m == 4) {
+    const uint32_t lane = lane_id();
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * 4;
+    for (uint64_t w0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x - lane) * 4; w0 < nseg; w0 += stride) {
+        const uint64_t s0 = w0 + lane * 4;
+        bool ones = skip_single && s0 + 4 <= nseg;
+        uint32_t first = 0;
+        if (ones) {
             const uint4 w = *reinterpret_cast<const uint4 *>(seg_start + s0);
-            at[0] = w.x; at[1] = w.y; at[2] = w.z; at[3] = w.w;
-            at[4] = seg_start[s0 + 4];
-            if (skip_single && at[1] - at[0] == 1 && at[2] - at[1] == 1 && at[3] - at[2] == 1 && at[4] - at[3] == 1) {
-                if (mark_starts) {
-#pragma unroll
-                    for (uint32_t k = 0; k < 4; ++k) b.flags[at[0] + k] = 1;
-                }
-                continue;
-            }
-        } else {
-#pragma unroll
-            for (uint32_t k = 0; k < 5; ++k) at[k] = k <= m ? seg_start[s0 + k] : 0u;
+            first = w.x;
+            // (starts increase but for empty segments)
+            ones = w.y - w.x == 1 && w.z - w.y == 1 && w.w - w.z == 1 && seg_start[s0 + 4] - w.w == 1;
         }
+        if (__all_sync(0xFFFFFFFFu, ones)) {
+            if (mark_starts) {
 #pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) b.flags[first + k] = 1;
+            }
+            continue;
+        }
+#pragma unroll 1
         for (uint32_t k = 0; k < 4; ++k) {
-            if (k >= m) break;
-            const uint32_t start = at[k], len = at[k + 1] - at[k];
+            const uint64_t s = w0 + k * 32 + lane;
+            if (s >= nseg) break;
+            const uint32_t start = seg_start[s], len = seg_start[s + 1] - start;
             if (mark_starts && len) b.flags[start] = 1;
             if (len == 1) {
                 // A one-row segment keeps its position.  With skip_single its

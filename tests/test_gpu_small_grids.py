@@ -18,3 +18,40 @@ def test_plain_rounds_by_chunk(ctx, n, dtype, bits):
     ng = ctx.sort_round_plain(bank, bits, order, out_group=group)
     o, g, _, ng_ref = O.sort_round(bank)
     assert ng == ng_ref and np.array_equal(order, o) and np.array_equal(group, g)
+
+
+@pytest.mark.parametrize("nseg", [127, 128, 129, 255, 256, 131, 4 * 256 * 148 + 5])
+@pytest.mark.parametrize("kind", ["ones", "one pair last", "pairs", "mixed"])
+def test_segments_by_warp(ctx, nseg, kind):
+    """The classification's steps of 128 segments a warp: all of one row, one that
+    is not, none that are; several rounds of a plan and a batch."""
+    rng = np.random.default_rng(nseg)
+    sizes = np.ones(nseg, np.int64)
+    if kind == "one pair last":
+        sizes[-1] = 2
+    elif kind == "pairs":
+        sizes[:] = 2
+    elif kind == "mixed":
+        sizes = rng.choice([1, 1, 1, 1, 2, 3, 17, 40], size=nseg)
+    n = int(sizes.sum())
+    first = rng.permutation(np.repeat(np.arange(nseg), sizes)).astype(np.uint32)
+    cols = [first, rng.integers(0, 3, size=n).astype(np.uint16), rng.integers(0, 5, size=n).astype(np.uint16)]
+    bw = split = [20, 2, 3]
+    o, g, ng_ref = O.run_plan_sort(cols, bw, split)
+    order, group = np.zeros(n, np.uint32), np.zeros(n, np.uint32)
+    assert ctx.run_plan(cols, bw, split, order, group) == ng_ref
+    assert np.array_equal(order, o) and np.array_equal(group, g)
+    if n > 1000:
+        counts = ctx.run_batch(cols, bw, split, [n], order, group)
+        assert counts[0] == ng_ref and np.array_equal(order, o) and np.array_equal(group, g)
+    # the instances themselves as segments, most of one row
+    few = sizes[:3000]
+    n = int(few.sum())
+    cols = [c[:n].copy() for c in cols[1:]]
+    order, group = np.zeros(n, np.uint32), np.zeros(n, np.uint32)
+    ctx.run_batch(cols, [2, 3], [2, 3], few, order, group)
+    off = 0
+    for size in few[:300]:
+        o, g, _ = O.run_plan_sort([c[off:off + size].copy() for c in cols], [2, 3], [2, 3])
+        assert np.array_equal(order[off:off + size], o) and np.array_equal(group[off:off + size], g)
+        off += size
