@@ -68,15 +68,29 @@ constexpr int pow2_ceil(int x)
 
 // (off is accessed by 16-byte vectors, and the warps of a CTA have an array of
 // these: both alignments are stated, whatever the members before)
+// What only skewed segments need lies where the compounds go: as long as they are
+// bucketed anew the rows' compounds are in registers.  Shared memory that is not
+// used is L1, which holds the sectors in flight of a later round's random key
+// reads: with these arrays beside cs a round of 16M rows in random order took 515
+// us in segments of 2048 rows and 703 in segments of 2200, with them in it 454 and
+// 502.
 template <typename K, int NT, int IT>
 struct alignas(16) OnchipSmem {
     static constexpr int kRows = NT * IT;
     static constexpr int kBins = pow2_ceil(kRows) < 128 ? 128 : pow2_ceil(kRows);
-    unsigned long long cs[kRows];   // compounds, bucketed
-    unsigned long long spl[NT];     // sorted splitters
-    uint32_t cst[NT];               // per coarse bucket: its start
-    float cinv[NT];                 // and its rows per unit of compound
-    uint32_t lowest[kRows / 16 + 1], highest[kRows / 16 + 1];   // per large bucket (its start / 16): its sampled range
+    struct Ranges {
+        uint32_t lowest[kRows / 16 + 1], highest[kRows / 16 + 1];   // per large bucket (its start / 16): its sampled range
+    };
+    struct Splitters {
+        unsigned long long spl[NT];   // sorted splitters
+        uint32_t cst[NT];             // per coarse bucket: its start
+        float cinv[NT];               // and its rows per unit of compound
+    };
+    union {
+        unsigned long long cs[kRows];   // compounds, bucketed
+        Ranges rg;
+        Splitters sp;
+    };
     uint32_t vals[kRows];           // oids by position
     alignas(16) uint32_t off[kBins + 4];   // per bucket: count -> start; then len
     unsigned long long any[NT / 32], all[NT / 32];   // per warp: OR and AND of its keys
@@ -292,13 +306,14 @@ __device__ __forceinline__ uint32_t splitter_place(uint32_t t, uint32_t len)
 }
 
 // The splitters of step 1's second try: NT compounds of the segment (in sm.cs
-// by position), sorted into sm.spl.  Out of line: it runs for skewed segments
+// by position), sorted into sm.sp.spl, which takes sm.cs's place.  Out of line: it runs for skewed segments
 // only, and its registers must not weigh on the others.
 template <typename K, int NT, int IT>
 __device__ __noinline__ void sort_splitters(OnchipSmem<K, NT, IT> &sm, uint32_t len, uint32_t drop, uint32_t nbits)
 {
     const uint32_t tid = NT == 32 ? lane_id() : threadIdx.x;
     unsigned long long x = sm.cs[splitter_place<NT>(tid, len)];
+    group_sync<NT>();   // the splitters go where the compounds were
 #pragma unroll 1
     for (uint32_t k = 2; k <= (uint32_t)NT; k <<= 1) {
 #pragma unroll 1
@@ -307,16 +322,16 @@ __device__ __noinline__ void sort_splitters(OnchipSmem<K, NT, IT> &sm, uint32_t 
             if (j < 32) {
                 y = __shfl_xor_sync(0xFFFFFFFFu, x, j);
             } else {
-                sm.spl[tid] = x;
+                sm.sp.spl[tid] = x;
                 group_sync<NT>();
-                y = sm.spl[tid ^ j];
+                y = sm.sp.spl[tid ^ j];
                 group_sync<NT>();
             }
             const bool lower = ((tid & k) == 0) == ((tid & j) == 0);
             x = comp_less(sm, y, x, drop, nbits) == lower ? y : x;
         }
     }
-    sm.spl[tid] = x;
+    sm.sp.spl[tid] = x;
 }
 
 // The compounds in sm.cs sorted in place, len of them, 2^nbits >= len: a bitonic
@@ -447,8 +462,8 @@ __device__ __forceinline__ OnchipInfo onchip_core(OnchipSmem<K, NT, IT> &sm, uns
         // large buckets: cut by the 32 bits after the digit, interpolated between
         // the lowest and the highest that one row a thread shows
         for (uint32_t i = tid; i <= len / 16; i += NT) {
-            sm.lowest[i] = 0xFFFFFFFFu;
-            sm.highest[i] = 0u;
+            sm.rg.lowest[i] = 0xFFFFFFFFu;
+            sm.rg.highest[i] = 0u;
         }
         if (tid == 0) sm.maxb = 0;
         group_sync<NT>();
@@ -464,8 +479,8 @@ __device__ __forceinline__ OnchipInfo onchip_core(OnchipSmem<K, NT, IT> &sm, uns
                 bk[j] = bs | (m << 16);
                 if (j == 0 && m >= 16u) {
                     const uint32_t d = next32(c[j]);
-                    atomicMin(&sm.lowest[bs >> 4], d);
-                    atomicMax(&sm.highest[bs >> 4], d);
+                    atomicMin(&sm.rg.lowest[bs >> 4], d);
+                    atomicMax(&sm.rg.highest[bs >> 4], d);
                 }
             }
         }
@@ -479,7 +494,7 @@ __device__ __forceinline__ OnchipInfo onchip_core(OnchipSmem<K, NT, IT> &sm, uns
                 uint32_t fb = bk[j] & 0xFFFFu;
                 const uint32_t m = bk[j] >> 16;
                 if (m >= 16u) {
-                    const uint32_t a = sm.lowest[fb >> 4], z = sm.highest[fb >> 4], d = next32(c[j]);
+                    const uint32_t a = sm.rg.lowest[fb >> 4], z = sm.rg.highest[fb >> 4], d = next32(c[j]);
                     // (no row sampled: a > z, everything goes to the first)
                     if (d > a && z > a) {
                         const float f = (float)(d - a) * __fdividef((float)m, (float)(z - a));
@@ -511,7 +526,7 @@ __device__ __forceinline__ OnchipInfo onchip_core(OnchipSmem<K, NT, IT> &sm, uns
                 uint32_t bi = 0;
 #pragma unroll 1
                 for (uint32_t h = NT / 2; h > 0; h >>= 1)
-                    if (!comp_less(sm, c[j], sm.spl[bi + h], drop, nbits)) bi += h;
+                    if (!comp_less(sm, c[j], sm.sp.spl[bi + h], drop, nbits)) bi += h;
                 bk[j] = bi;
                 atomicAdd(&sm.off[bi], 1u);
             }
@@ -521,12 +536,12 @@ __device__ __forceinline__ OnchipInfo onchip_core(OnchipSmem<K, NT, IT> &sm, uns
         // interpolation leaves it out)
         const unsigned long long cmask = drop ? ~(unsigned long long)pmask : ~0ull;
         {
-            const unsigned long long a = tid ? sm.spl[tid] & cmask : 0ull;
-            const unsigned long long z = tid + 1 < (uint32_t)NT ? sm.spl[tid + 1] & cmask
+            const unsigned long long a = tid ? sm.sp.spl[tid] & cmask : 0ull;
+            const unsigned long long z = tid + 1 < (uint32_t)NT ? sm.sp.spl[tid + 1] & cmask
                                                                 : ~0ull >> (64u - (top - drop) - nbits);
             const uint32_t s0 = sm.off[tid];
-            sm.cst[tid] = s0;
-            sm.cinv[tid] = (float)(sm.off[tid + 1] - s0) / ((float)(z - a) + 1.0f);
+            sm.sp.cst[tid] = s0;
+            sm.sp.cinv[tid] = (float)(sm.off[tid + 1] - s0) / ((float)(z - a) + 1.0f);
         }
         group_sync<NT>();
         zero_bins<NT>(sm.off, NT == 32 && nb < 128 ? 128u : nb, tid);
@@ -537,15 +552,20 @@ __device__ __forceinline__ OnchipInfo onchip_core(OnchipSmem<K, NT, IT> &sm, uns
             const uint32_t p = wbase + j * 32 + lane;
             if (j < (int)steps && p < len) {
                 const uint32_t bi = bk[j];
-                const unsigned long long a = bi ? sm.spl[bi] & cmask : 0ull;
-                const uint32_t s0 = sm.cst[bi];
-                const uint32_t e0 = bi + 1 < (uint32_t)NT ? sm.cst[bi + 1] : len;
-                const uint32_t f = (uint32_t)(__ull2float_rn((c[j] & cmask) - a) * sm.cinv[bi]);
+                const unsigned long long a = bi ? sm.sp.spl[bi] & cmask : 0ull;
+                const uint32_t s0 = sm.sp.cst[bi];
+                const uint32_t e0 = bi + 1 < (uint32_t)NT ? sm.sp.cst[bi + 1] : len;
+                const uint32_t f = (uint32_t)(__ull2float_rn((c[j] & cmask) - a) * sm.sp.cinv[bi]);
                 const uint32_t fb = s0 + min(f, e0 - s0 - 1u);
                 bk[j] = (fb << 16) | atomicAdd(&sm.off[fb], 1u);
             }
         }
         if (group_scan_bins<K, NT, IT>(sm, nb, len) > kBucketWorst) {   // (uniform across the group)
+#pragma unroll
+            for (int j = 0; j < IT; ++j) {
+                const uint32_t p = wbase + j * 32 + lane;
+                if (j < (int)steps && p < len) sm.cs[p] = c[j];
+            }
             sort_network<K, NT, IT>(sm, len, drop, nbits);
             return OnchipInfo{prefix, nbits, drop, false};
         }
