@@ -55,3 +55,26 @@ def test_segments_by_warp(ctx, nseg, kind):
         o, g, _ = O.run_plan_sort([c[off:off + size].copy() for c in cols], [2, 3], [2, 3])
         assert np.array_equal(order[off:off + size], o) and np.array_equal(group[off:off + size], g)
         off += size
+
+
+@pytest.mark.parametrize("n", [1, 2, 16, 17, 33, 129, 257, 513, 1025, 2049, 2305, 4097, 8192, 8193])
+@pytest.mark.parametrize("values", [1, 2, 1 << 20])
+def test_small_hash_plans(ctx, n, values):
+    """Clustering sorts that fit one tier, one value among them; eager and captured."""
+    import torch
+    rng = np.random.default_rng(n)
+    cols = [rng.integers(0, values, size=n).astype(np.uint32), rng.integers(0, 3, size=n).astype(np.uint16),
+            rng.integers(0, 2, size=n).astype(np.uint16)]
+    bw = split = [20, 2, 1]
+    o, g, ng_ref = O.run_plan_hash(cols, bw, split)
+    order, group = np.zeros(n, np.uint32), np.zeros(n, np.uint32)
+    assert ctx.run_plan(cols, bw, split, order, group, hash=True) == ng_ref
+    assert np.array_equal(order, o) and np.array_equal(group, g)
+    dev = [torch.from_numpy(c.view({2: np.int16, 4: np.int32}[c.itemsize])).cuda() for c in cols]
+    d_order, d_group = (torch.zeros(n, dtype=torch.int32, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    graph = ctx.plan_graph(dev, bw, split, d_order, d_group, hash=True)
+    assert graph.launch() == ng_ref
+    assert np.array_equal(d_order.cpu().numpy().view(np.uint32), o)
+    assert np.array_equal(d_group.cpu().numpy().view(np.uint32), g)
+    graph.close()
