@@ -40,6 +40,17 @@ struct StitchParams {
 
 constexpr int kStitchCtas = 4;   // resident CTAs per SM
 
+// Rows of a group of four, and where a lane's groups start.  VEC: neighbours,
+// moved by vectors.  Else (some array off a 16-byte boundary) 32 apart, so that a
+// warp's lanes still read and write neighbours: the 32 groups of a warp hold its
+// 128 rows either way.  (Four neighbours a lane, one access each: 16M rows of
+// 1 + 2 + 4 bytes into 4 took 117 us, 79 so.)
+template <bool VEC>
+struct Group4 {
+    static constexpr uint32_t kStep = VEC ? 1u : 32u;
+    static __device__ __forceinline__ uint64_t first_row(uint64_t g) { return VEC ? g * 4 : (g & ~31ull) * 4 + (g & 31u); }
+};
+
 // Four rows of one slice as they come from memory: MAXB (the widest source's
 // bytes per row) words.
 template <int MAXB>
@@ -48,28 +59,34 @@ struct Raw4 {
 };
 
 // VEC: one vector load (the rows are whole and the source is aligned); else
-// row by row, zero past n.
+// row by row (Group4), zero past n.
 template <int MAXB, bool VEC>
 __device__ __forceinline__ void load_raw(const void *base, uint32_t bytes, uint64_t row, uint64_t n, Raw4<MAXB> &r)
 {
     if constexpr (!VEC) {
+        // (the width is looked at once, so that the four loads are in flight together)
+        auto four = [&](auto *p, auto &&put) {
 #pragma unroll
-        for (int i = 0; i < MAXB; ++i) r.w[i] = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (row + k >= n) break;
-            if (bytes == 8) {
-                const uint64_t v = ((const uint64_t *)base)[row + k];
-                if constexpr (MAXB >= 8) {
+            for (int k = 0; k < 4; ++k) {
+                const uint64_t at = row + k * Group4<VEC>::kStep;
+                put(k, at < n ? p[at] : 0u);
+            }
+        };
+        if (bytes == 8) {
+            if constexpr (MAXB >= 8)
+                four((const uint64_t *)base, [&](int k, uint64_t v) {
                     r.w[2 * k] = (uint32_t)v;
                     r.w[2 * k + 1] = (uint32_t)(v >> 32);
-                }
-            } else if (bytes == 4) {
-                if constexpr (MAXB >= 4) r.w[k] = ((const uint32_t *)base)[row + k];
-            } else if (bytes == 2) {
-                r.w[k >> 1] |= (uint32_t)((const uint16_t *)base)[row + k] << (16 * (k & 1));
+                });
+        } else if (bytes == 4) {
+            if constexpr (MAXB >= 4) four((const uint32_t *)base, [&](int k, uint32_t v) { r.w[k] = v; });
+        } else {
+            r.w[0] = 0;
+            if (bytes == 2) {
+                r.w[1] = 0;
+                four((const uint16_t *)base, [&](int k, uint32_t v) { r.w[k >> 1] |= v << (16 * (k & 1)); });
             } else {
-                r.w[0] |= (uint32_t)((const uint8_t *)base)[row + k] << (8 * k);
+                four((const uint8_t *)base, [&](int k, uint32_t v) { r.w[0] |= v << (8 * k); });
             }
         }
         return;
@@ -161,8 +178,10 @@ __device__ __forceinline__ void store4(B *bank, uint64_t row, uint64_t n, const 
         }
     } else {
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (row + k < n) bank[row + k] = (B)a[k];
+        for (int k = 0; k < 4; ++k) {
+            const uint64_t at = row + k * Group4<VEC>::kStep;
+            if (at < n) bank[at] = (B)a[k];
+        }
     }
 }
 
@@ -191,7 +210,7 @@ __global__ void __launch_bounds__(256, kStitchCtas) stitch_kernel(const __grid_c
     kernel_prologue();
     constexpr int kBatch = MAXB == 8 ? 1 : MAXB == 4 ? 3 : 4;
     __shared__ uint32_t sh[2][256];
-    const uint64_t groups = VEC ? n / 4 : (n + 3) / 4;
+    const uint64_t groups = VEC ? n / 4 : (n + 127) / 128 * 32;
     auto count = [&](const uint64_t (&a)[4], uint64_t row, uint32_t *hist) {
         uint32_t d[4];
         if (hist_lo >= 32) {
@@ -203,11 +222,12 @@ __global__ void __launch_bounds__(256, kStitchCtas) stitch_kernel(const __grid_c
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (VEC || row + k < n) atomicAdd(&hist[d[k] & hist_mask], 1u);
+            if (VEC || row + k * Group4<VEC>::kStep < n) atomicAdd(&hist[d[k] & hist_mask], 1u);
     };
     auto step = [&](uint64_t g, uint64_t stride, uint64_t g_end, uint32_t *hist) {
         const bool two = g + stride < g_end;
-        const uint64_t row0 = g * 4, row1 = (two ? g + stride : g) * 4;   // (a lone group is folded twice)
+        // (a lone group is folded twice)
+        const uint64_t row0 = Group4<VEC>::first_row(g), row1 = Group4<VEC>::first_row(two ? g + stride : g);
         uint64_t a0[4] = {0, 0, 0, 0}, a1[4] = {0, 0, 0, 0};
 #pragma unroll 1
         for (int s0 = 0; s0 < p.ns; s0 += kBatch) {
@@ -403,7 +423,7 @@ int launch_stitch(fmcs_ctx *ctx, const StitchSlice *sl, int ns, void *bank, uint
     LaunchScope ls_(ctx, "stitch");
     auto launch = [&](auto *b) {
         using B = std::remove_pointer_t<decltype(b)>;
-        auto *k = !aligned    ? stitch_kernel<B, 8, false>
+        auto *k = !aligned    ? (maxb <= 4 ? stitch_kernel<B, 4, false> : stitch_kernel<B, 8, false>)
                   : maxb <= 2 ? stitch_kernel<B, 2, true>
                   : maxb <= 4 ? stitch_kernel<B, 4, true>
                               : stitch_kernel<B, 8, true>;

@@ -78,3 +78,29 @@ def test_small_hash_plans(ctx, n, values):
     assert np.array_equal(d_order.cpu().numpy().view(np.uint32), o)
     assert np.array_equal(d_group.cpu().numpy().view(np.uint32), g)
     graph.close()
+
+
+@pytest.mark.parametrize("n", [8193, 8193 + 127, 20_001, 300_001, 1_300_003])
+@pytest.mark.parametrize("widest", [4, 8])
+def test_plans_of_unaligned_columns(ctx, n, widest):
+    """Columns and outputs one element off a 16-byte boundary: bank and first-level
+    histogram from warps of 128 rows whose last are past the end."""
+    import torch
+    rng = np.random.default_rng(n)
+    bw = [12, 27] + ([40] if widest == 8 else [])
+    types = [np.uint16, np.uint32, np.uint64]
+    signed = {2: np.int16, 4: np.int32, 8: np.int64}
+    cols = [rng.integers(0, 1 << w, size=n, dtype=np.uint64).astype(t) for w, t in zip(bw, types)]
+    cols[0] %= 5
+    dev = []
+    for c in cols:
+        d = torch.from_numpy(np.concatenate([c[:1], c]).view(signed[c.itemsize])).cuda()
+        dev.append(d[1:])
+    order, group = (torch.full((n + 2,), -7, dtype=torch.int32, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    for split in ([sum(bw)] if sum(bw) <= 64 else [64, sum(bw) - 64], bw):
+        o, g, ng_ref = O.run_plan_sort(cols, bw, split)
+        assert ctx.run_plan(dev, bw, split, order[1:n + 1], group[1:n + 1]) == ng_ref
+        h_order, h_group = order.cpu().numpy(), group.cpu().numpy()
+        assert np.array_equal(h_order[1:n + 1].view(np.uint32), o) and np.array_equal(h_group[1:n + 1].view(np.uint32), g)
+        assert (h_order[[0, n + 1]] == -7).all() and (h_group[[0, n + 1]] == -7).all()
