@@ -31,6 +31,10 @@ from . import workloads as W
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 DEFAULT_OUT = os.path.join(HERE, "tuning", "b200.json")
+# Rows of the round whose time is a round's fixed cost: the fewest that do not
+# take the one-launch path of small rounds (8192 rows), which no round of a
+# larger plan takes.
+ROUND_FIXED_ROWS = 8193
 KNOBS = {"rank_mode": (0, 1, 2), "local_max": (2048, 4096, 8192), "msd_items": (8, 16)}
 
 
@@ -97,6 +101,17 @@ def search_knobs(ctx, wl: Workloads):
     return best, [{"ms": round(ms, 4), **kn} for ms, kn in results]
 
 
+def fixed_round(ctx):
+    """A call whose time is a round's fixed cost: device arrays, a radix level, one
+    on-chip tier and the group ids, with next to no rows."""
+    import torch
+    n = ROUND_FIXED_ROWS
+    bank = torch.arange(n - 1, -1, -1, dtype=torch.int32, device="cuda")
+    order, group = torch.empty_like(bank), torch.empty_like(bank)
+    torch.cuda.synchronize()
+    return lambda: ctx.sort_round(bank, 14, order, out_group=group)
+
+
 def calibrate(ctx, quick: bool) -> dict:
     import torch
     n = 1 << (22 if quick else 24)
@@ -150,9 +165,7 @@ def calibrate(ctx, quick: bool) -> dict:
     out["boundary"] = boundary
     out["msd_level"] = msd
     out["local"] = local
-    tiny = np.arange(1024, dtype=np.uint32)[::-1].copy()
-    to = np.zeros(1024, np.uint32)
-    out["round_fixed_ms"] = _time(lambda: ctx.sort_round(tiny, 10, to), 21)
+    out["round_fixed_ms"] = _time(fixed_round(ctx), 21)
     return out
 
 
