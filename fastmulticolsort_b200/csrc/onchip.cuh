@@ -305,6 +305,30 @@ __device__ __forceinline__ uint32_t splitter_place(uint32_t t, uint32_t len)
     return a + __umulhi(h, z - a);
 }
 
+// Rows of the bucket [bs, bs + bn) that sort before x, when the keys' low bits are
+// dropped from the compounds.  Another row with the same kept bits is rare: only
+// then do the dropped ones decide.  (A round over 16M rows of 64-bit keys in
+// segments of 2048: 405 us when every comparison looked at them, 356 so.  Out of
+// line, as its registers and instructions weigh on the segments that drop nothing:
+// the first radix round of 16M 50-bit keys 557 us with it inline, 544 without.)
+template <typename K, int NT, int IT>
+__device__ __noinline__ uint32_t rank_dropped(const OnchipSmem<K, NT, IT> &sm, uint32_t bs, uint32_t bn,
+                                              unsigned long long x, uint32_t drop, uint32_t nbits)
+{
+    const uint32_t pmask = (1u << nbits) - 1u;
+    uint32_t r = 0, same = 0;
+    for (uint32_t q = 0; q < bn; ++q) {
+        const unsigned long long y = sm.cs[bs + q];
+        r += y < x;
+        same += (y ^ x) <= pmask;
+    }
+    if (same > 1) {
+        r = 0;
+        for (uint32_t q = 0; q < bn; ++q) r += comp_less(sm, sm.cs[bs + q], x, drop, nbits);
+    }
+    return r;
+}
+
 // The splitters of step 1's second try: NT compounds of the segment (in sm.cs
 // by position), sorted into sm.sp.spl, which takes sm.cs's place.  Out of line: it runs for skewed segments
 // only, and its registers must not weigh on the others.
@@ -594,7 +618,7 @@ __device__ __forceinline__ OnchipInfo onchip_core(OnchipSmem<K, NT, IT> &sm, uns
             if (sizeof(K) < 8 || drop == 0) {
                 for (uint32_t q = 0; q < bn; ++q) r += sm.cs[bs + q] < c[j];
             } else {
-                for (uint32_t q = 0; q < bn; ++q) r += comp_less(sm, sm.cs[bs + q], c[j], drop, nbits);
+                r = rank_dropped(sm, bs, bn, c[j], drop, nbits);
             }
             bk[j] = (bs + r) | 0x80000000u;   // its place; it moves
         }
