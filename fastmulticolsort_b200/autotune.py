@@ -35,6 +35,8 @@ DEFAULT_OUT = os.path.join(HERE, "tuning", "b200.json")
 # take the one-launch path of small rounds (8192 rows), which no round of a
 # larger plan takes.
 ROUND_FIXED_ROWS = 8193
+# The kernels that sort a round's groups, by the names the profiler gives them.
+GROUP_SORT_KERNELS = ("thread_sort", "warp_sort", "block_sort", "copy", "classify", "msd_", "tile_prefix")
 KNOBS = {"rank_mode": (0, 1, 2), "local_max": (2048, 4096, 8192), "msd_items": (8, 16)}
 
 
@@ -157,8 +159,7 @@ def calibrate(ctx, quick: bool) -> dict:
             ctx.sort_round(src, bits, oo.clone(), in_group=ig, out_group=gg)
             prof = ctx.profile_report()
             ctx.profile(False)
-            lm = sum(v["ms"] for kk, v in prof.items()
-                     if kk.startswith(("warp_sort", "block_sort", "copy", "classify", "msd_", "tile_prefix")))
+            lm = sum(v["ms"] for kk, v in prof.items() if kk.startswith(GROUP_SORT_KERNELS))
             row.append(lm / mrows)
         local.append(row)
     out["gather"] = gather

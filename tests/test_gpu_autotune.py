@@ -22,3 +22,18 @@ def test_fixed_cost_of_a_round(ctx):
     ran = _ran(ctx, autotune.fixed_round(ctx))
     assert {"classify", "tile_prefix", "msd_hist", "msd_plan", "msd_scatter", "boundary_scan"} <= ran
     assert [k for k in ran if k.startswith(("thread_sort", "warp_sort", "block_sort"))]
+
+
+@pytest.mark.parametrize("size", [2, 8, 32, 128, 512, 8192])
+def test_group_sorts_are_counted(ctx, size):
+    """Every kernel between a segmented round's boundary scans is one of the group
+    sorts (and the hand-over of the counters)."""
+    import torch
+    n = 1 << 16
+    bank = torch.randint(0, 1 << 15, (n,), dtype=torch.int32, device="cuda")
+    in_group = torch.arange(n, dtype=torch.int32, device="cuda") // size
+    group = torch.empty_like(bank)
+    ran = _ran(ctx, lambda: ctx.sort_round(bank, 15, torch.arange(n, dtype=torch.int32, device="cuda"),
+                                           in_group=in_group, out_group=group))
+    assert {k for k in ran if not k.startswith(autotune.GROUP_SORT_KERNELS)} <= {"boundary_scan", "publish"}
+    assert [k for k in ran if k.startswith(("thread_sort", "warp_sort", "block_sort"))]
