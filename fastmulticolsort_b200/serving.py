@@ -94,7 +94,9 @@ def warm(torch, srv, pool, slots, rounds=1):
     device-wide synchronisation, on the latency of every request in flight):
     each request of the pool, largest first, submitted `slots` times at once so
     that every slot runs it; then the whole pool at once, so that the shared
-    launches of small requests are warm too."""
+    launches of small requests are warm too.  The pool's plans are searched for
+    before that: a search takes longer than a small request runs, and requests
+    that arrive a search apart share no launch.  Returns how many did."""
     for d in sorted(pool, key=lambda d: -d["n"]):
         keep = []
         for _ in range(slots):
@@ -102,13 +104,13 @@ def warm(torch, srv, pool, slots, rounds=1):
             keep.append((srv.submit(d["cols"], d["widths"], o, cardinality=d["card"]), o))
         for tk, _ in keep:
             srv.wait(tk)
+    splits = [capi.optimize_plan(d["widths"], d["card"], [c.element_size() for c in d["cols"]], d["n"])[0] for d in pool]
+    shared = 0
     for _ in range(rounds):
-        keep = []
-        for d in pool:
-            o = torch.empty(d["n"], dtype=torch.int32, device="cuda")
-            keep.append((srv.submit(d["cols"], d["widths"], o, cardinality=d["card"]), o))
-        for tk, _ in keep:
-            srv.wait(tk)
+        outs = [torch.empty(d["n"], dtype=torch.int32, device="cuda") for d in pool]
+        keep = [srv.submit(d["cols"], d["widths"], o, split=s) for d, o, s in zip(pool, outs, splits)]
+        shared += sum(srv.wait(tk)["batched_with"] > 1 for tk in keep)
+    return shared
 
 
 def run_served(torch, srv, pool, trace, slots, keep=None):

@@ -52,3 +52,16 @@ def test_burst_on_one_host_core():
         o, g, _ = O.run_plan_sort(cols, bw, [17, 33])
         assert np.array_equal(order.cpu().numpy().view(np.uint32), o)
         assert np.array_equal(group.cpu().numpy().view(np.uint32), g)
+
+
+def test_serving_warm_up_shares_launches():
+    """The warm-up leaves the shared launches' workspace grown: it has to make some."""
+    import torch
+    from fastmulticolsort_b200 import capi, serving
+    rng = np.random.default_rng(4)
+    pool = []
+    for n in rng.integers(60_000, 300_000, size=24):
+        cols = [serving._store(torch, serving._uniform_codes(torch, rng, int(n), w), w) for w in (8, 24, 40)]
+        pool.append(dict(n=int(n), widths=[8, 24, 40], cols=cols, card=[min(int(n), 1 << w) for w in (8, 24, 40)]))
+    with capi.Server(0, slots=4, batch_rows_max=1 << 20) as server:
+        assert serving.warm(torch, server, pool, 4) > len(pool) // 4
