@@ -119,8 +119,13 @@ int sort_round_dev(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, uint32_
 
 // Plans of fewer rows than this find their groups by a scan of the sorted keys:
 // flags save 14 bytes a row of traffic (8-byte keys) and cost the on-chip sorts
-// some instructions and a store.  16.8M rows [50] 634 us by keys, 621 by flags;
-// 384 instances (38.6M rows) 2.78 and 2.68 ms; but 90,001 rows 174 and 183.
+// some instructions and a store.  Keys and flags, us: 131,072 rows [50] 88 and 86,
+// [19] 82 and 84; 1M [50] 128 and 126, [17,33] 178 and 173; 8.4M [17,33] 479 and
+// 456; 16.8M [50] 634 and 621.  From about 1M rows flags gain 1 to 5%, below it the
+// two are within 3% either way.  (Batches take flags at any size: their instances
+// are given by their starts, with no group vector for a scan of keys to read.
+// fmcs_sort_round never does: it is given the group vector, and may be asked for
+// the sorted keys.)
 constexpr uint64_t kFlagRows = 1ull << 20;
 
 // The group-start flags of n rows (every sort round writes what it splits).

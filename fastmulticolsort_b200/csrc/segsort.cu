@@ -91,7 +91,7 @@ constexpr int kCtrWords = kHostCounterWords;
 // digit bases running on in registers.  Every kSuper chunks of a segment also
 // share a super row, the sum of theirs, so that no plan CTA walks more than
 // kSuper chunk rows and a few super rows.
-// Chunk size: one tile as long as there are no more than 32,768 (each is flushed
+// Chunk size: one tile as long as there are fewer than 32,768 (each is flushed
 // and planned).  Larger chunks cost: the scatter's last round over its 444
 // resident CTAs is as long as a chunk, and neighbouring tiles, whose rows share
 // the ends of every digit's run, are then written far apart in time, so that

@@ -9,9 +9,11 @@
 // it goes, and a segmented round sorts by its bank and then by its segment.
 // Group ids are an adjacent difference over the banks and one scan.
 // Bound: latency, one SM's barriers and shared memory.  3,001 rows, one 50-bit
-// bank: 10 us in this kernel, 36 us the call (48 with eight launches); 5,588
-// rows in banks of 64 and 2 bits: 77 us (91).  The limit is what one CTA's
-// shared memory holds; at 8,192 rows one launch still wins.
+// bank: 10 us in this kernel, 26 us the call (41 by the general path's launches).
+// The limit is what one CTA's shared memory holds.  There, at 8,192 rows, one
+// launch against the general path: [50] 38 us (49), [17,33] 57 (83), [64,20] 82
+// (100), six columns in [59,7] 84 (86); only three rounds driven one by one lose,
+// 188 (180).
 #include "device_common.cuh"
 #include "fmcs_internal.h"
 #include "onchip.cuh"
@@ -227,13 +229,14 @@ int launch_small_t(fmcs_ctx *ctx, const SmallParams &p, const char *name)
     return e == cudaSuccess ? FMCS_OK : cuda_fail(ctx, e, "small plan launch");
 }
 
-int launch_small(fmcs_ctx *ctx, const SmallParams &p)
+int launch_small(fmcs_ctx *ctx, const SmallParams &p, bool plan)
 {
     // as few rows a thread as the block allows: the steps are a serial chain
-    // (profiled under the name of the on-chip tier of that capacity)
-    return p.n <= 1024   ? launch_small_t<256, 4>(ctx, p, "block_sort_1024")
-           : p.n <= 4096 ? launch_small_t<1024, 4>(ctx, p, "block_sort_4096")
-                         : launch_small_t<1024, 8>(ctx, p, "block_sort_8192");
+    // (profiled as a plan by its own name; as a round under the name of the
+    // on-chip tier of that capacity, the one sort of a segment that it is)
+    return p.n <= 1024   ? launch_small_t<256, 4>(ctx, p, plan ? "small_plan" : "block_sort_1024")
+           : p.n <= 4096 ? launch_small_t<1024, 4>(ctx, p, plan ? "small_plan" : "block_sort_4096")
+                         : launch_small_t<1024, 8>(ctx, p, plan ? "small_plan" : "block_sort_8192");
 }
 
 }  // namespace
@@ -261,7 +264,7 @@ int launch_small_plan(fmcs_ctx *ctx, const StitchSlice *slices, const int *nslic
     p.order_out = order_out;
     p.group_out = group_out;
     p.d_ngroups = d_ngroups;
-    return launch_small(ctx, p);
+    return launch_small(ctx, p, true);
 }
 
 int launch_small_round(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, uint32_t key_bits, const uint32_t *order_in,
@@ -280,7 +283,7 @@ int launch_small_round(fmcs_ctx *ctx, const void *bank, uint32_t bank_bytes, uin
     p.keys_out = keys_out;
     p.key_bytes = bank_bytes;
     p.d_ngroups = group_out ? d_ngroups : nullptr;
-    return launch_small(ctx, p);
+    return launch_small(ctx, p, false);
 }
 
 }  // namespace fmcs

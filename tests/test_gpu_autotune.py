@@ -37,3 +37,12 @@ def test_group_sorts_are_counted(ctx, size):
                                            in_group=in_group, out_group=group))
     assert {k for k in ran if not k.startswith(autotune.GROUP_SORT_KERNELS)} <= {"boundary_scan", "publish"}
     assert [k for k in ran if k.startswith(("thread_sort", "warp_sort", "block_sort"))]
+
+
+@pytest.mark.parametrize("n", [100, 1025, 8192])
+def test_small_plans_go_by_their_name(ctx, n):
+    """The profiler reports a small plan's one launch as that, not as a tier."""
+    import torch
+    col = torch.arange(n, dtype=torch.int32, device="cuda")
+    order, group = torch.empty_like(col), torch.empty_like(col)
+    assert _ran(ctx, lambda: ctx.run_plan([col], [20], [12, 8], order, group)) == {"small_plan"}
