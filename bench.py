@@ -503,6 +503,10 @@ def run_fmcs(args):
     launches = (ctx.launch_count() - lc0) // max(1, args.steps) * args.steps
     prof = {k: v for k, v in ctx.profile_report().items() if not k.startswith("_")}
     ctx.profile(False)
+    if not args.only_steps:
+        # an eager step's time is taken without the events (and with the tiers
+        # on both streams, as a user's call has them)
+        eager_total, _ = time_steps(ctx, stream, step, args.steps)
     eager_ms = dist_max(eager_total / args.steps, world)
     if args.only_steps:
         graph.close()
