@@ -38,7 +38,7 @@ namespace {
 // position bits find a row's oid when the segment is written out, so only
 // compounds move.
 //
-// Bound: issue slots and shared-memory latency, about 100 instructions a row
+// Bound: issue slots and shared-memory latency, about 230 instructions a row
 // (the HBM traffic is 24 bytes a row for 8-byte keys).  A warp sorts a segment of
 // up to 256 rows by itself: no block barriers, and three to four times as many
 // rows in flight per SM as one small CTA per segment.  (One warp for 512 rows
