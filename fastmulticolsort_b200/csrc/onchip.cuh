@@ -305,28 +305,66 @@ __device__ __forceinline__ uint32_t splitter_place(uint32_t t, uint32_t len)
     return a + __umulhi(h, z - a);
 }
 
+// The dropped low bits and the position of a compound, as one word.
+template <typename K, int NT, int IT>
+__device__ __forceinline__ uint32_t low_word(const OnchipSmem<K, NT, IT> &sm, unsigned long long x, uint32_t nbits)
+{
+    const uint32_t p = (uint32_t)x & ((1u << nbits) - 1u);
+    return ((uint32_t)sm.lo[p] << nbits) | p;
+}
+
 // Rows of the bucket [bs, bs + bn) that sort before x, when the keys' low bits are
-// dropped from the compounds.  Another row with the same kept bits is rare: only
-// then do the dropped ones decide.  (A round over 16M rows of 64-bit keys in
-// segments of 2048: 405 us when every comparison looked at them, 356 so.  Out of
-// line, as its registers and instructions weigh on the segments that drop nothing:
-// the first radix round of 16M 50-bit keys 557 us with it inline, 544 without.)
+// dropped from the compounds.  As long as no other row with the same kept bits is
+// met (spread-out keys: hardly ever), the compounds decide; then the count starts
+// again and looks at the dropped bits of such rows.  (A round over 16M rows of
+// 64-bit keys in segments of 2048: 405 us when every comparison looked at them, 336
+// so; 2.4M rows of 200 values in segments of 2000 186 us and 144.  Out of line, as
+// its registers and instructions weigh on the segments that drop nothing: the first
+// radix round of 16M 50-bit keys 557 us with it inline, 544 without.)
 template <typename K, int NT, int IT>
 __device__ __noinline__ uint32_t rank_dropped(const OnchipSmem<K, NT, IT> &sm, uint32_t bs, uint32_t bn,
-                                              unsigned long long x, uint32_t drop, uint32_t nbits)
+                                              unsigned long long x, uint32_t nbits)
 {
     const uint32_t pmask = (1u << nbits) - 1u;
     uint32_t r = 0, same = 0;
-    for (uint32_t q = 0; q < bn; ++q) {
+    for (uint32_t q = 0; q < bn && same < 2u; ++q) {
         const unsigned long long y = sm.cs[bs + q];
         r += y < x;
         same += (y ^ x) <= pmask;
     }
-    if (same > 1) {
+    if (same > 1u) {
+        const uint32_t xl = low_word(sm, x, nbits);
         r = 0;
-        for (uint32_t q = 0; q < bn; ++q) r += comp_less(sm, sm.cs[bs + q], x, drop, nbits);
+        for (uint32_t q = 0; q < bn; ++q) {
+            const unsigned long long y = sm.cs[bs + q];
+            r += (y ^ x) <= pmask ? low_word(sm, y, nbits) < xl : y < x;
+        }
     }
     return r;
+}
+
+// The fine bucket of x among the m rows of coarse bucket bi, when the keys' low
+// bits are dropped: by the kept bits (inv rows per unit of compound), or, where
+// they are the same in both its splitters, by dropped bits and position.
+// (Otherwise the rows of a key that is frequent enough to be many splitters would
+// share a fine bucket: a round over 2.4M 64-bit keys of 16 values in segments of
+// 8000 rows 449 us, 285 so.)  Out of line, as rank_dropped is.
+template <typename K, int NT, int IT>
+__device__ __noinline__ uint32_t fine_dropped(const OnchipSmem<K, NT, IT> &sm, uint32_t bi, uint32_t m, float inv,
+                                              unsigned long long x, uint32_t nbits)
+{
+    const uint32_t pmask = (1u << nbits) - 1u;
+    const unsigned long long a = bi ? sm.sp.spl[bi] : 0ull;
+    if (bi && bi + 1 < (uint32_t)NT) {
+        const unsigned long long z = sm.sp.spl[bi + 1];
+        if ((a ^ z) <= pmask) {
+            const uint32_t al = low_word(sm, a, nbits);
+            const float span = (float)(low_word(sm, z, nbits) - al) + 1.0f;
+            return min((uint32_t)((float)(low_word(sm, x, nbits) - al) * __fdividef((float)m, span)), m - 1u);
+        }
+    }
+    const unsigned long long kept = ~(unsigned long long)pmask;
+    return min((uint32_t)(__ull2float_rn((x & kept) - (a & kept)) * inv), m - 1u);
 }
 
 // The splitters of step 1's second try: NT compounds of the segment (in sm.cs
@@ -576,11 +614,15 @@ __device__ __forceinline__ OnchipInfo onchip_core(OnchipSmem<K, NT, IT> &sm, uns
             const uint32_t p = wbase + j * 32 + lane;
             if (j < (int)steps && p < len) {
                 const uint32_t bi = bk[j];
-                const unsigned long long a = bi ? sm.sp.spl[bi] & cmask : 0ull;
                 const uint32_t s0 = sm.sp.cst[bi];
                 const uint32_t e0 = bi + 1 < (uint32_t)NT ? sm.sp.cst[bi + 1] : len;
-                const uint32_t f = (uint32_t)(__ull2float_rn((c[j] & cmask) - a) * sm.sp.cinv[bi]);
-                const uint32_t fb = s0 + min(f, e0 - s0 - 1u);
+                uint32_t fb = s0;
+                if (sizeof(K) == 8 && drop) {
+                    fb += fine_dropped(sm, bi, e0 - s0, sm.sp.cinv[bi], c[j], nbits);
+                } else {
+                    const unsigned long long a = bi ? sm.sp.spl[bi] : 0ull;
+                    fb += min((uint32_t)(__ull2float_rn(c[j] - a) * sm.sp.cinv[bi]), e0 - s0 - 1u);
+                }
                 bk[j] = (fb << 16) | atomicAdd(&sm.off[fb], 1u);
             }
         }
@@ -618,7 +660,7 @@ __device__ __forceinline__ OnchipInfo onchip_core(OnchipSmem<K, NT, IT> &sm, uns
             if (sizeof(K) < 8 || drop == 0) {
                 for (uint32_t q = 0; q < bn; ++q) r += sm.cs[bs + q] < c[j];
             } else {
-                r = rank_dropped(sm, bs, bn, c[j], drop, nbits);
+                r = rank_dropped(sm, bs, bn, c[j], nbits);
             }
             bk[j] = (bs + r) | 0x80000000u;   // its place; it moves
         }

@@ -87,3 +87,23 @@ def test_skewed_segments_take_no_longer_than_a_network(ctx, kind, rows):
             times.append(sum(v["ms"] for name, v in prof.items() if name.startswith("block_sort")))
         best[k] = min(times[1:])
     assert 0 < best[kind] < 10 * best["random"], best
+
+
+@pytest.mark.parametrize("values", [2, 16, 200, 3000])
+@pytest.mark.parametrize("zipf", [False, True])
+@pytest.mark.parametrize("bits", [50, 60, 64])
+def test_few_values(ctx, bits, zipf, values):
+    """Segments of every tier whose keys are a few long codes: rows of one key are
+    told apart by their positions, beside dropped low bits or next to the key."""
+    rng = np.random.default_rng(values + bits)
+    codes = rng.integers(0, (1 << bits) - 1, size=values, dtype=np.uint64, endpoint=True)
+    codes[1] = codes[0] ^ np.uint64(1)   # the same but for the last bit
+    p = 1.0 / np.arange(1, values + 1) if zipf else np.ones(values)
+    sizes = [s - d for s in sorted(TIERS) for d in (0, 1, 40)] + [128, 130, 20_000]
+    bank = codes[rng.choice(values, size=sum(sizes), p=p / p.sum())]
+    in_group = np.repeat(np.arange(len(sizes), dtype=np.uint32), sizes)
+    order_in = rng.permutation(bank.shape[0]).astype(np.uint32)
+    order, group, keys = order_in.copy(), np.zeros_like(order_in), np.zeros_like(bank)
+    ng = ctx.sort_round(bank, bits, order, in_group=in_group, out_group=group, sorted_bank=keys)
+    o, g, k, ng_ref = O.sort_round(bank, order=order_in, in_group=in_group)
+    assert ng == ng_ref and np.array_equal(order, o) and np.array_equal(group, g) and np.array_equal(keys, k)
